@@ -292,6 +292,12 @@ __device__ __forceinline__ void drain_tile(const GArgs &a, uint32_t acc, uint32_
             load_chunk_bf16(a.gu + row_g * a.N + h0, g);
             load_chunk_bf16(a.gu + row_g * a.N + a.H + h0, u);
             tmem_ld_wait();
+            if (!valid) {
+                // a padding row of kept pre-activations is whatever the forward call found in its workspace; its
+                // products must be zeros (the weight gradients contract over all rows of the block), not 0 * NaN
+#pragma unroll
+                for (int j = 0; j < 32; ++j) c[j] = g[j] = u[j] = 0.f;
+            }
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 const float s = 1.f / (1.f + __expf(-g[j]));

@@ -165,6 +165,23 @@ def test_kept_pre_activations(T, K, E, N, k, bpc):
     check(tuple(g.cpu() for g in grads), O.moe_backward_ref_fp32(x, w1, w2, ids, wts, d_out))
 
 
+@pytest.mark.parametrize("fill", [float("nan"), float("inf")])
+def test_padding_rows_of_kept_pre_activations_do_not_reach_the_gradients(fill):
+    """Padding rows of the kept gate | up buffer hold whatever the forward call's workspace held: here NaN / Inf."""
+    from prime_flash_moe_b200 import capi
+    T, K, E, N, k = 70, 256, 4, 512, 2
+    x, w1, w2, ids, wts = O.make_case(T, K, E, N, k, seed=19)
+    d_out = torch.randn(T, K, generator=torch.Generator().manual_seed(3)).to(torch.bfloat16)
+    s, e, n = capi.moe_align(ids.to(DEV), E, 128, 1)
+    dx, dw1, dw2, dwts = x.to(DEV), w1.to(DEV), w2.to(DEV), wts.to(DEV)
+    _, gate_up = capi.fused_moe_bf16_keep(dx, dw1, dw2, s, e, n, dwts, torch.empty_like(dx), k)
+    gate_up[s < 0] = fill
+    grads = capi.fused_moe_bf16_backward(dx, dw1, dw2, d_out.to(DEV), s, e, n, dwts, k, gate_up=gate_up)
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    check(tuple(g.cpu() for g in grads), O.moe_backward_ref_fp32(x, w1, w2, ids, wts, d_out))
+
+
 @pytest.mark.parametrize("recompute", [False, True])
 def test_autograd_layer_matches_oracle_gradients(recompute):
     import prime_flash_moe_b200 as P
