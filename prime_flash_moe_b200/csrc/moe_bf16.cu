@@ -420,10 +420,9 @@ moe_up_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const uint32_t fill_bytes =
                 a.pregathered == 2 ? B_BYTES : (short_a ? B_BYTES + SHORT_A_BYTES : STAGE_BYTES);
             for (int ks = 0; ks < ksteps; ++ks) {
-                if (lane == 0) ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+                ok = __all_sync(0xffffffffu, mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY));
                 if (!ok) break;
-                if (lane == 0) {
+                if (elect_one()) {
                     mbar_arrive_expect_tx(sm.full(s), fill_bytes);
                     tma_load_2d(sm.b(s), &map_w1, sm.full(s), ks * BK, row_gate);
                     tma_load_2d(sm.b(s) + B_BYTES / 2, &map_w1, sm.full(s), ks * BK, row_up);
@@ -448,7 +447,7 @@ moe_up_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(128, 256);
             int s = 0;
             uint32_t ph = 0;
@@ -691,7 +690,7 @@ moe_up_dual_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
 
     if (warp == 0) {
         // ---------------- producer: weight slots (and the pre-gathered A tiles) by TMA ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -725,7 +724,7 @@ moe_up_dual_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(128, 256);
             int s = 0;
             uint32_t ph = 0;
@@ -954,7 +953,7 @@ moe_down_bf16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_c
     const int num_tiles = base_tiles * ksplit;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             long long issued = 0;
@@ -984,7 +983,7 @@ moe_down_bf16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_c
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(128, 256);
             int s = 0;
             uint32_t ph = 0;
@@ -1121,10 +1120,9 @@ moe_fused_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             const int row_gate = e * a.N + c.n_tile * 128;
             const int row_up = row_gate + a.H;
             for (int ks = 0; ks < ksteps; ++ks) {
-                if (lane == 0) ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+                ok = __all_sync(0xffffffffu, mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY));
                 if (!ok) break;
-                if (lane == 0) {
+                if (elect_one()) {
                     mbar_arrive_expect_tx(sm.full(s), STAGE_BYTES);
                     tma_load_2d(sm.b(s), &map_w1, sm.full(s), ks * BK, row_gate);
                     tma_load_2d(sm.b(s) + B_BYTES / 2, &map_w1, sm.full(s), ks * BK, row_up);
@@ -1147,10 +1145,9 @@ moe_fused_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             // down phase: w2[e][chunk*128 .. +128, slice*128 + kh*64 .. +64] -> B part of a slot
             for (int ch = 0; ch < dn_chunks && ok; ++ch) {
                 for (int kh = 0; kh < 2; ++kh) {
-                    if (lane == 0) ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
+                    ok = __all_sync(0xffffffffu, mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY));
                     if (!ok) break;
-                    if (lane == 0) {
+                    if (elect_one()) {
                         mbar_arrive_expect_tx(sm.full(s), B_BYTES / 2);
                         tma_load_2d(sm.b(s), &map_w2, sm.full(s), c.n_tile * 128 + kh * 64, e * a.K + ch * 128);
                     }
@@ -1165,7 +1162,7 @@ moe_fused_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         if (!ok && lane == 0) drain_fills(sm, a.stages, issued);
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_up = idesc_bf16_f32(128, 256);
             constexpr uint32_t idesc_dn = idesc_bf16_f32(128, 128);
             int s = 0;
@@ -1354,7 +1351,7 @@ moe_pair_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int first = blockIdx.x >> 1, step = gridDim.x >> 1;   // this pair's tile sequence
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -1368,7 +1365,7 @@ moe_pair_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 if (kUp) b_row = e * a.N + c.n_tile * 128 + (leader ? 0 : a.H);
                 else b_row = e * a.K + c.n_tile * 256 + static_cast<int>(rank) * 128;
                 for (int ks = 0; ks < ksteps; ++ks) {
-                    ok = mbar_wait_cluster(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
+                    ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
                     if (!ok) break;
                     const uint32_t full_leader = mapa_shared(sm.full(s), 0);
                     if (leader) mbar_arrive_expect_tx(sm.full(s), 2 * PAIR_STAGE_BYTES);
@@ -1383,7 +1380,7 @@ moe_pair_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader && elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(256, 256);
             int s = 0;
             uint32_t ph = 0;
@@ -1396,7 +1393,7 @@ moe_pair_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 tc_fence_after();
                 const uint32_t d = tmem_base + buf * 256;
                 for (int ks = 0; ks < ksteps; ++ks) {
-                    ok = mbar_wait_cluster(sm.full(s), ph, status, ST_TIMEOUT_FULL);
+                    ok = mbar_wait(sm.full(s), ph, status, ST_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll

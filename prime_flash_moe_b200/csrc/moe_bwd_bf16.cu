@@ -426,7 +426,7 @@ moe_bwd_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int num_tiles = a_mn ? a.E * a.m_tiles * a.n_tiles : m_items * a.n_tiles;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             long long issued = 0;
@@ -473,7 +473,7 @@ moe_bwd_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(BM, BN) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
             int s = 0;
             uint32_t ph = 0;
@@ -627,7 +627,7 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int first = blockIdx.x >> 1, step = gridDim.x >> 1;   // this pair's tile sequence
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -637,7 +637,7 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const int blk = tl.mb + static_cast<int>(rank);                 // row space: this CTA's row block
                 const int n0 = tl.nt * BN + static_cast<int>(rank) * 128;       // this CTA's N indices of B
                 for (int ks = tl.k0; ks < tl.k1; ++ks) {
-                    ok = mbar_wait_cluster(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
+                    ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
                     if (!ok) break;
                     const uint32_t full_leader = mapa_shared(sm.full(s), 0);
                     if (leader) mbar_arrive_expect_tx(sm.full(s), 2 * PAIR_STAGE_BYTES);
@@ -665,7 +665,7 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader && elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(256, 256) | (wgrad ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
             int s = 0;
             uint32_t ph = 0;
@@ -680,7 +680,7 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 tc_fence_after();
                 const uint32_t d = tmem_base + buf * BN;
                 for (int ks = tl.k0; ks < tl.k1; ++ks) {
-                    ok = mbar_wait_cluster(sm.full(s), ph, status, ST_TIMEOUT_FULL);
+                    ok = mbar_wait(sm.full(s), ph, status, ST_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll

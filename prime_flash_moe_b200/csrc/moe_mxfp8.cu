@@ -252,7 +252,7 @@ moe_up_mxfp8_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const int ksteps = a.K / BKB;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             long long issued = 0;
@@ -291,7 +291,7 @@ moe_up_mxfp8_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_mxf8_f32(128, 256);
             int s = 0;
             uint32_t ph = 0;
@@ -487,7 +487,7 @@ moe_down_mxfp8_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_
     const int ksteps = a.H / BKB;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             long long issued = 0;
@@ -520,7 +520,7 @@ moe_down_mxfp8_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_mxf8_f32(128, 256);
             int s = 0;
             uint32_t ph = 0;
@@ -691,7 +691,7 @@ moe_pair_mxfp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int first = blockIdx.x >> 1, step = gridDim.x >> 1;   // this pair's tile sequence
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -714,7 +714,7 @@ moe_pair_mxfp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 }
                 const int sfa0 = blk * ksteps;
                 for (int ks = 0; ks < ksteps; ++ks) {
-                    ok = mbar_wait_cluster(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
+                    ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
                     if (!ok) break;
                     const uint32_t full_leader = mapa_shared(sm.full(s), 0);
                     if (leader) mbar_arrive_expect_tx(sm.full(s), 2 * PAIR_TX_BYTES);
@@ -732,7 +732,7 @@ moe_pair_mxfp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader && elect_one()) {
             constexpr uint32_t idesc = idesc_mxf8_f32(256, 256);
             int s = 0;
             uint32_t ph = 0;
@@ -744,7 +744,7 @@ moe_pair_mxfp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 if (!ok) break;
                 tc_fence_after();
                 for (int ks = 0; ks < ksteps; ++ks, ++fill) {
-                    ok = mbar_wait_cluster(sm.full(s), ph, status, ST_TIMEOUT_FULL);
+                    ok = mbar_wait(sm.full(s), ph, status, ST_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t sfa_t = tmem_base + SF_TMEM_BASE + 16u * static_cast<uint32_t>(fill & 7);
@@ -937,7 +937,7 @@ moe_fused_mxfp8_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     const int dn_chunks = a.K / 128;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             long long issued = 0;
@@ -986,7 +986,7 @@ moe_fused_mxfp8_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_up = idesc_mxf8_f32(128, 256);
             constexpr uint32_t idesc_dn = idesc_mxf8_f32(128, 128);
             int s = 0;

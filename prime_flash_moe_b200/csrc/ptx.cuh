@@ -53,7 +53,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
-// one elected lane of a converged warp
+// One elected lane of a converged warp. The TMA producer and MMA issuer loops run under `if (elect_one())`, not under
+// `if (lane == 0)`: the compiler knows that an elect.sync branch has exactly one active thread and keeps the operands
+// of cp.async.bulk.tensor / tcgen05.mma (descriptors, coordinates, barrier addresses) in uniform registers, while
+// under a lane comparison every such instruction pays for moving them there. Measured on a 2048 x 9472 x K grouped
+// GEMM with CTA pairs (256 x 256 tiles, six 64-wide k-steps in flight): 0.44 us per k-step with the comparison, 0.36
+// with elect (0.33 with the loads left out, i.e. the MMAs themselves).
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(
@@ -360,7 +365,9 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
         : "memory");
     return ok != 0;
 }
-// bounded wait on a barrier whose arrivals may come from the peer CTA
+// Bounded wait on a barrier on which threads of the peer CTA arrive (accumulator hand-back: once per tile). The ring
+// barriers of the pair kernels complete through TMA bytes and tcgen05.commit, not through another thread's writes:
+// they take the plain mbar_wait (a cluster-scope acquire per k-step made the same GEMM 10 % slower).
 static __device__ __noinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int *status, int code) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
