@@ -26,8 +26,11 @@ namespace {
 
 constexpr int kWarpsPerCta = 8;
 constexpr int kThreads = kWarpsPerCta * 32;
-constexpr int kSmallN = 4096;      // up to here a single CTA of 8 warps does everything, no scratch
-constexpr int kSmallN32 = 16384;   // ... and up to here a single CTA of 32 warps, when its counters fit (E <= 256)
+constexpr int kOneCtaN = 2048;     // up to here a single CTA does everything, no scratch
+// Without scratch memory a single CTA also takes up to kSmallN ids (8 warps) or kSmallN32 (32 warps, E <= 256), at
+// 2.2 us per 1000 ids: 8192 ids, E = 128: 23 us on one CTA, 9 us on several; 16384 ids: 39 and 10 us.
+constexpr int kSmallN = 4096;
+constexpr int kSmallN32 = 16384;
 constexpr int kMaxExperts = 1024;
 
 __device__ __forceinline__ unsigned lanemask_lt() {
@@ -38,7 +41,7 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 
 // Count the ids of [begin, end) into cnt[0..E) (private to the calling warp, already zeroed).
 // Four 32-id groups are loaded ahead of their match rounds so that the loads overlap.
-__device__ __forceinline__ void warp_histogram(const int32_t *__restrict__ ids, int begin, int end, int E,
+__device__ __forceinline__ void warp_histogram(const int32_t *ids, int begin, int end, int E,
                                                int *cnt) {
     const int lane = threadIdx.x & 31;
     for (int base = begin; base < end; base += 128) {
@@ -46,7 +49,7 @@ __device__ __forceinline__ void warp_histogram(const int32_t *__restrict__ ids, 
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int i = base + 32 * u + lane;
-            v[u] = (i < end) ? __ldg(ids + i) : -1;
+            v[u] = (i < end) ? ids[i] : -1;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -62,7 +65,7 @@ __device__ __forceinline__ void warp_histogram(const int32_t *__restrict__ ids, 
 }
 
 // Replay [begin, end): cur[e] is this warp's next write position for expert e.
-__device__ __forceinline__ void warp_scatter(const int32_t *__restrict__ ids, int begin, int end, int E,
+__device__ __forceinline__ void warp_scatter(const int32_t *ids, int begin, int end, int E,
                                              int *cur, int32_t *__restrict__ sorted, int max_padded) {
     const int lane = threadIdx.x & 31;
     for (int base = begin; base < end; base += 128) {
@@ -70,7 +73,7 @@ __device__ __forceinline__ void warp_scatter(const int32_t *__restrict__ ids, in
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int i = base + 32 * u + lane;
-            v[u] = (i < end) ? __ldg(ids + i) : -1;
+            v[u] = (i < end) ? ids[i] : -1;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -148,10 +151,10 @@ __device__ void block_offsets(const int *tot, int *offs, int *wsum, int E, int p
 // ---------------------------------------------------------------------------------------------
 // small n: one CTA, no scratch
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) moe_align_small_kernel(
-    const int32_t *__restrict__ ids, int32_t *__restrict__ sorted, int32_t *__restrict__ expert_ids,
-    int32_t *__restrict__ npp, int n, int E, int block_m, int pad_to, int max_padded, int max_blocks) {
-    extern __shared__ int sm[];
+// `ids` may lie in global or in shared memory; `sm` holds (warps + 2) * E + 1 + warps ints
+__device__ __forceinline__ void align_one_cta(const int32_t *ids, int *sm, int32_t *__restrict__ sorted,
+                                              int32_t *__restrict__ expert_ids, int32_t *__restrict__ npp, int n, int E,
+                                              int block_m, int pad_to, int max_padded, int max_blocks) {
     const int nthr = blockDim.x, nwarps = nthr >> 5;   // 8 warps, or 32 for the larger single-CTA problems
     int *cnt = sm;                 // [nwarps][E]
     int *tot = cnt + nwarps * E;   // [E]
@@ -196,6 +199,15 @@ __global__ void __launch_bounds__(1024) moe_align_small_kernel(
     warp_scatter(ids, begin, end, E, cnt + warp * E, sorted, max_padded);
 }
 
+__global__ void __launch_bounds__(1024) moe_align_small_kernel(
+    const int32_t *__restrict__ ids, int32_t *__restrict__ sorted, int32_t *__restrict__ expert_ids,
+    int32_t *__restrict__ npp, int n, int E, int block_m, int pad_to, int max_padded, int max_blocks) {
+    extern __shared__ int sm[];
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the router, when launched as its programmatic dependent
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    align_one_cta(ids, sm, sorted, expert_ids, npp, n, E, block_m, pad_to, max_padded, max_blocks);
+}
+
 // ---------------------------------------------------------------------------------------------
 // general n: two launches. The ids are cut into one contiguous segment per CTA (and per warp inside it).
 //   histogram kernel   per-warp private counters in shared memory -> counts[cta][e] (coalesced), and the
@@ -237,7 +249,7 @@ __global__ void __launch_bounds__(kThreads) moe_align_hist_kernel(
 __global__ void __launch_bounds__(kThreads) moe_align_scatter_kernel(
     const int32_t *__restrict__ ids, int n, int E, int seg, const int *__restrict__ counts, int block_m,
     int pad_to, int32_t *__restrict__ sorted, int32_t *__restrict__ expert_ids, int32_t *__restrict__ npp,
-    int max_padded, int max_blocks, int ids_from_primary) {
+    int max_padded, int max_blocks) {
     extern __shared__ int sm[];
     int *cnt = sm;                       // [kWarpsPerCta][E] per-warp counts, later per-warp write cursors
     int *tot = cnt + kWarpsPerCta * E;   // [E] ids of expert e in all CTAs
@@ -249,10 +261,9 @@ __global__ void __launch_bounds__(kThreads) moe_align_scatter_kernel(
     __syncthreads();
     const int gw = blockIdx.x * kWarpsPerCta + warp;
     const int begin = min(gw * seg, n), end = min(begin + seg, n);
-    // after the fused router the ids themselves come from the preceding kernel: wait before reading them
-    if (ids_from_primary) asm volatile("griddepcontrol.wait;" ::: "memory");
     warp_histogram(ids, begin, end, E, cnt + warp * E);
     asm volatile("griddepcontrol.wait;" ::: "memory");   // the histogram kernel's counts and -1 fill are complete
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // column sums of counts[cta][e]: `parts` threads share one expert when there are fewer experts than threads
     const int ctas = gridDim.x, me = blockIdx.x;
     const int parts = max(1, kThreads / E);
@@ -295,17 +306,27 @@ struct Plan {
     size_t ws_ints; // scratch ints: counts[ctas][E]
 };
 
-constexpr int kIdsPerCtaMin = 2048;
+constexpr int kIdsPerCtaMin = 2048;        // every CTA reads the counters of all: few large segments ...
+constexpr int kIdsPerCtaMinShort = 512;    // ... but not so few that a short problem leaves the chip idle
 
 Plan make_plan(int n, int E) {
     Plan p{};
-    if (n <= kSmallN || (n <= kSmallN32 && E <= 256)) return p;
-    int ctas = (n + kIdsPerCtaMin - 1) / kIdsPerCtaMin;
+    if (n <= kOneCtaN) return p;
+    const int per_cta = n <= kSmallN32 ? kIdsPerCtaMinShort : kIdsPerCtaMin;
+    int ctas = (n + per_cta - 1) / per_cta;
     ctas = std::max(1, std::min(ctas, sm_count()));
     p.ctas = ctas;
     const int warps = ctas * kWarpsPerCta;
     p.seg = ((n + warps - 1) / warps + 31) & ~31;
     p.ws_ints = static_cast<size_t>(E) * ctas;
+    return p;
+}
+
+// the plan of a call whose scratch may be missing or short: short problems then run on one CTA
+Plan plan_with_scratch(int n, int E, const void *workspace, size_t workspace_bytes) {
+    const Plan p = make_plan(n, E);
+    if ((!workspace || workspace_bytes < p.ws_ints * sizeof(int)) && (n <= kSmallN || (n <= kSmallN32 && E <= 256)))
+        return Plan{};
     return p;
 }
 
@@ -329,33 +350,40 @@ int check_args(const void *topk_ids, const void *sorted, const void *expert_ids,
 
 int launch(const int32_t *topk_ids, int32_t *sorted, int32_t *expert_ids, int32_t *npp, int n, int E,
            int block_m, int pad_to, int max_padded, int max_blocks, const Plan &p, int *ws,
-           cudaStream_t stream) {
+           cudaStream_t stream, bool after_router = false) {
+    // Right after the router's launch the one-CTA kernel is its programmatic dependent: it waits for it before it reads
+    // an id, only its launch overlaps. The histogram kernel is not: the scatter kernel starts with it and counts the
+    // ids beside it, so the router has to be complete by then (T = 8192, E = 128: 33 us with the scatter kernel waiting).
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = after_router && pdl_enabled() ? 1 : 0;
     if (p.ctas == 0) {
         const int warps = n > 1024 && E <= 256 ? 32 : kWarpsPerCta;
         const size_t smem = (static_cast<size_t>(warps) * E + 2 * E + 1 + warps) * sizeof(int);   // <= 35 KB
-        moe_align_small_kernel<<<1, warps * 32, smem, stream>>>(topk_ids, sorted, expert_ids, npp, n, E, block_m,
-                                                             pad_to, max_padded, max_blocks);
-        PMOE_CUDA_OK(cudaGetLastError());
+        cfg.gridDim = dim3(1);
+        cfg.blockDim = dim3(warps * 32);
+        cfg.dynamicSmemBytes = smem;
+        PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_align_small_kernel, topk_ids, sorted, expert_ids, npp, n, E, block_m,
+                                        pad_to, max_padded, max_blocks));
         return PMOE_OK;
     }
     int *counts = ws;
     const size_t smem_h = static_cast<size_t>(kWarpsPerCta) * E * sizeof(int);
-    moe_align_hist_kernel<<<p.ctas, kThreads, smem_h, stream>>>(topk_ids, n, E, p.seg, counts, sorted, max_padded);
-    PMOE_CUDA_OK(cudaGetLastError());
-    const size_t smem_s = (static_cast<size_t>(kWarpsPerCta) * E + 3 * static_cast<size_t>(E) + 1 + kWarpsPerCta) *
-                          sizeof(int);
-    cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ctas);
     cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_h;
+    cfg.numAttrs = 0;
+    PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_align_hist_kernel, topk_ids, n, E, p.seg, counts, sorted, max_padded));
+    const size_t smem_s = (static_cast<size_t>(kWarpsPerCta) * E + 3 * static_cast<size_t>(E) + 1 + kWarpsPerCta) *
+                          sizeof(int);
     cfg.dynamicSmemBytes = smem_s;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
     PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_align_scatter_kernel, topk_ids, n, E, p.seg, static_cast<const int *>(counts),
-                                    block_m, pad_to, sorted, expert_ids, npp, max_padded, max_blocks, 0));
+                                    block_m, pad_to, sorted, expert_ids, npp, max_padded, max_blocks));
     return PMOE_OK;
 }
 
@@ -363,66 +391,61 @@ int launch(const int32_t *topk_ids, int32_t *sorted, int32_t *expert_ids, int32_
 }  // namespace pmoe
 
 // ---------------------------------------------------------------------------------------------
-// router fused with the histogram pass: one kernel routes the tokens (softmax + top-k, one warp per token,
-// route_warp.cuh), writes topk_ids / topk_weights, counts its own ids per expert and fills sorted_token_ids with
-// -1 - i.e. it replaces route_topk_kernel AND moe_align_hist_kernel, and the ids are not read back for counting.
-// CTA c owns the ids [c*8*seg, (c+1)*8*seg) of the align plan, i.e. 8*seg / top_k whole tokens (the entry point
-// falls back to the two separate kernels when top_k does not divide 8*seg). 32 warps per CTA: the grid is the
-// align plan's (<= #SMs CTAs), so the tokens of a CTA are spread over more warps than the histogram pass has.
+// router + moe_align in one call
 // ---------------------------------------------------------------------------------------------
 namespace pmoe {
 namespace {
 
+// Decode batches: one CTA routes the tokens (one warp each, one or two rounds) and aligns the ids it still holds in
+// shared memory. T = 16, E = 128, top_k = 8: router 3.2 us + align 5.0 us + the gap between them 2.7 us before.
+constexpr int kOneCtaTokens = 32;      // one round of 32 warps (E <= 256); with 8 warps a quarter of it
+constexpr int kOneCtaExperts = 768;    // counters + ids fit 48 KB of shared memory
+
 template <typename T, int PER>
-__global__ void __launch_bounds__(1024) route_hist_kernel(
+__global__ void __launch_bounds__(1024) route_align_one_cta_kernel(
     const T *__restrict__ logits, int tokens, int E, int top_k, int renormalize, int32_t *__restrict__ topk_ids,
-    float *__restrict__ topk_weights, int tokens_per_cta, int *__restrict__ counts, int32_t *__restrict__ sorted,
-    int max_padded) {
-    extern __shared__ int s_cnt[];   // [E]
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (int e = threadIdx.x; e < E; e += blockDim.x) s_cnt[e] = 0;
-    __syncthreads();
+    float *__restrict__ topk_weights, int32_t *__restrict__ sorted, int32_t *__restrict__ expert_ids,
+    int32_t *__restrict__ npp, int block_m, int pad_to, int max_padded, int max_blocks) {
+    extern __shared__ int sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int t0 = blockIdx.x * tokens_per_cta, t1 = min(tokens, t0 + tokens_per_cta);
-    for (int t = t0 + warp; t < t1; t += nwarps) {
+    int32_t *ids = sm + (nwarps + 2) * E + 1 + nwarps;   // [tokens * top_k]
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (int t = warp; t < tokens; t += nwarps) {
         int idx;
         float w;
         route_token_warp<T, PER>(logits + static_cast<size_t>(t) * E, E, top_k, renormalize, lane, idx, w);
         if (lane < top_k) {
+            ids[t * top_k + lane] = idx;
             topk_ids[static_cast<size_t>(t) * top_k + lane] = idx;
             topk_weights[static_cast<size_t>(t) * top_k + lane] = w;
-            atomicAdd(&s_cnt[idx], 1);   // shared-memory integer counts: independent of the order of the adds
         }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) counts[static_cast<size_t>(blockIdx.x) * E + e] = s_cnt[e];
-    int4 *s4 = reinterpret_cast<int4 *>(sorted);
-    const int n4 = max_padded >> 2;
-    const int4 m1 = make_int4(-1, -1, -1, -1);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) s4[i] = m1;
-    if (blockIdx.x == 0 && threadIdx.x < (max_padded & 3)) sorted[(n4 << 2) + threadIdx.x] = -1;
+    align_one_cta(ids, sm, sorted, expert_ids, npp, tokens * top_k, E, block_m, pad_to, max_padded, max_blocks);
 }
 
 template <typename T>
-int launch_route_hist(const T *logits, int tokens, int E, int top_k, int renormalize, int32_t *ids, float *wts,
-                      const Plan &p, int *counts, int32_t *sorted, int max_padded, cudaStream_t stream) {
-    const int tokens_per_cta = kWarpsPerCta * p.seg / top_k;
-    const size_t smem = static_cast<size_t>(E) * sizeof(int);
+int launch_route_align_one_cta(const T *logits, int tokens, int E, int top_k, int renormalize, int32_t *ids, float *wts,
+                               int32_t *sorted, int32_t *expert_ids, int32_t *npp, int block_m, int pad_to,
+                               int max_padded, int max_blocks, cudaStream_t stream) {
+    const int warps = E <= 256 ? 32 : kWarpsPerCta;
+    const size_t smem = (static_cast<size_t>(warps + 2) * E + 1 + warps + static_cast<size_t>(tokens) * top_k) * sizeof(int);
     const int per = (E + 31) / 32;
-#define PMOE_ROUTE_HIST_CASE(P)                                                                                      \
+#define PMOE_ROUTE_ALIGN_CASE(P)                                                                                     \
     if (per <= P) {                                                                                                  \
-        route_hist_kernel<T, P><<<p.ctas, 1024, smem, stream>>>(logits, tokens, E, top_k, renormalize, ids, wts,     \
-                                                               tokens_per_cta, counts, sorted, max_padded);         \
+        route_align_one_cta_kernel<T, P><<<1, warps * 32, smem, stream>>>(logits, tokens, E, top_k, renormalize, ids, \
+                                                                         wts, sorted, expert_ids, npp, block_m,      \
+                                                                         pad_to, max_padded, max_blocks);            \
         PMOE_CUDA_OK(cudaGetLastError());                                                                            \
         return PMOE_OK;                                                                                              \
     }
-    PMOE_ROUTE_HIST_CASE(1)
-    PMOE_ROUTE_HIST_CASE(2)
-    PMOE_ROUTE_HIST_CASE(4)
-    PMOE_ROUTE_HIST_CASE(8)
-    PMOE_ROUTE_HIST_CASE(16)
-    PMOE_ROUTE_HIST_CASE(32)
-#undef PMOE_ROUTE_HIST_CASE
+    PMOE_ROUTE_ALIGN_CASE(1)
+    PMOE_ROUTE_ALIGN_CASE(2)
+    PMOE_ROUTE_ALIGN_CASE(4)
+    PMOE_ROUTE_ALIGN_CASE(8)
+    PMOE_ROUTE_ALIGN_CASE(16)
+    PMOE_ROUTE_ALIGN_CASE(32)
+#undef PMOE_ROUTE_ALIGN_CASE
     return set_error(PMOE_ERR_UNSUPPORTED, "route_topk_align supports at most 1024 experts, got %d", E);
 }
 
@@ -441,43 +464,27 @@ extern "C" int pmoe_route_topk_align(const void *logits, int logits_dtype, int T
     if (int rc = check_args(topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, n, num_experts, block_m,
                             pad_to, max_padded, max_blocks))
         return rc;
-    const Plan p = make_plan(n, num_experts);
+    const Plan p = plan_with_scratch(n, num_experts, workspace, workspace_bytes);
     PMOE_REQUIRE(p.ws_ints == 0 || (workspace && workspace_bytes >= p.ws_ints * sizeof(int)), PMOE_ERR_BAD_ARG,
                  "route_topk_align: workspace of %zu bytes required, got %zu", p.ws_ints * sizeof(int), workspace_bytes);
-    const bool fused = p.ctas > 0 && (kWarpsPerCta * p.seg) % top_k == 0 && logits && topk_weights && top_k <= 32 &&
-                       top_k <= num_experts && num_experts <= kMaxExperts &&
-                       (logits_dtype == PMOE_DTYPE_F32 || logits_dtype == PMOE_DTYPE_BF16);
-    if (!fused) {   // small problems (one CTA aligns them) and top_k that does not divide a CTA's id range
-        if (int rc = pmoe_route_topk(logits, logits_dtype, T, num_experts, top_k, renormalize, topk_ids, topk_weights,
-                                     stream))
-            return rc;
-        return launch(topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, n, num_experts, block_m, pad_to,
-                      max_padded, max_blocks, p, static_cast<int *>(workspace), stream);
-    }
-    int *counts = static_cast<int *>(workspace);
-    int rc = logits_dtype == PMOE_DTYPE_F32
-                 ? launch_route_hist(static_cast<const float *>(logits), T, num_experts, top_k, renormalize ? 1 : 0,
-                                     topk_ids, topk_weights, p, counts, sorted_token_ids, max_padded, stream)
-                 : launch_route_hist(static_cast<const __nv_bfloat16 *>(logits), T, num_experts, top_k,
-                                     renormalize ? 1 : 0, topk_ids, topk_weights, p, counts, sorted_token_ids,
-                                     max_padded, stream);
-    if (rc) return rc;
-    const size_t smem_s = (static_cast<size_t>(kWarpsPerCta) * num_experts + 3 * static_cast<size_t>(num_experts) + 1 +
-                           kWarpsPerCta) * sizeof(int);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.ctas);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem_s;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_align_scatter_kernel, static_cast<const int32_t *>(topk_ids), n, num_experts,
-                                    p.seg, static_cast<const int *>(counts), block_m, pad_to, sorted_token_ids, expert_ids,
-                                    num_tokens_post_padded, max_padded, max_blocks, 1));
-    return PMOE_OK;
+    const bool router_ok = logits && topk_weights && top_k <= 32 && top_k <= num_experts &&
+                           (logits_dtype == PMOE_DTYPE_F32 || logits_dtype == PMOE_DTYPE_BF16);
+    if (router_ok && p.ctas == 0 && T > 0 && num_experts <= kOneCtaExperts &&
+        T <= (num_experts <= 256 ? kOneCtaTokens : kOneCtaTokens / 4))
+        return logits_dtype == PMOE_DTYPE_F32
+                   ? launch_route_align_one_cta(static_cast<const float *>(logits), T, num_experts, top_k,
+                                                renormalize ? 1 : 0, topk_ids, topk_weights, sorted_token_ids, expert_ids,
+                                                num_tokens_post_padded, block_m, pad_to, max_padded, max_blocks, stream)
+                   : launch_route_align_one_cta(static_cast<const __nv_bfloat16 *>(logits), T, num_experts, top_k,
+                                                renormalize ? 1 : 0, topk_ids, topk_weights, sorted_token_ids, expert_ids,
+                                                num_tokens_post_padded, block_m, pad_to, max_padded, max_blocks, stream);
+    // The router on its own grid, one warp per token, then the align launches. (A router that also counts its ids runs
+    // on the align plan's grid, at most one CTA per 2048 ids: T = 8192, E = 128, top_k = 8 38 us against 18; T = 65536
+    // 104 against 64.)
+    if (int rc = pmoe_route_topk(logits, logits_dtype, T, num_experts, top_k, renormalize, topk_ids, topk_weights, stream))
+        return rc;
+    return launch(topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, n, num_experts, block_m, pad_to,
+                  max_padded, max_blocks, p, static_cast<int *>(workspace), stream, T > 0 && p.ctas == 0);
 }
 
 extern "C" size_t pmoe_moe_align_workspace_bytes(int n, int num_experts) {
@@ -493,7 +500,7 @@ extern "C" int pmoe_moe_align_ws(const int32_t *topk_ids, int32_t *sorted_token_
     if (int rc = check_args(topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, n, num_experts,
                             block_m, pad_to, max_padded, max_blocks))
         return rc;
-    const Plan p = make_plan(n, num_experts);
+    const Plan p = plan_with_scratch(n, num_experts, workspace, workspace_bytes);
     PMOE_REQUIRE(p.ws_ints == 0 || (workspace && workspace_bytes >= p.ws_ints * sizeof(int)), PMOE_ERR_BAD_ARG,
                  "moe_align: workspace of %zu bytes required, got %zu", p.ws_ints * sizeof(int),
                  workspace_bytes);

@@ -33,6 +33,7 @@ template <typename T, int PER>
 __global__ void __launch_bounds__(kRouteWarps * 32)
 route_topk_kernel(const T *__restrict__ logits, int tokens, int E, int top_k, int renormalize,
                   int32_t *__restrict__ topk_ids, float *__restrict__ topk_weights) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // an align kernel may set itself up meanwhile
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * kRouteWarps + (threadIdx.x >> 5);
     if (t >= tokens) return;

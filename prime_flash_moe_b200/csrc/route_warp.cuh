@@ -1,5 +1,5 @@
 // One warp routes one token: softmax + top-k over E router logits held in registers (lane l holds logits l, l+32,
-// ...). Shared by the stand-alone router kernel and by the router fused with the moe_align histogram pass.
+// ...). Shared by the stand-alone router kernel and by the one-CTA kernel that routes and aligns a decode batch.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -27,9 +27,61 @@ __device__ __forceinline__ float key_float(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+// top-k of one token for PER <= 8 logits per lane, none of them NaN: every lane sorts its own logits once (stable, so
+// that ties keep the lower index first); a round is a warp maximum over the heads, and its owner (of several, the one
+// with the lowest index) moves its list up by one. Returns false, with nothing selected, when fewer than
+// top_k logits are above -inf: the general loop below then decides.
+// Against the general loop (8192 tokens, E = 128, top_k = 8): router 23 -> 8 us.
+template <typename T, int PER>
+__device__ __forceinline__ bool select_sorted(const float (&v)[PER], int E, int top_k, int lane, float &my_val, int &my_idx,
+                                              float &row_max) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr uint32_t kMinusInf = 0x007fffffu;    // float_key(-inf); emptied slots and e >= E hold 0
+    uint32_t key[PER];
+    int idx[PER];
+    bool nan = false;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        idx[i] = lane + 32 * i;
+        key[i] = idx[i] < E ? float_key(v[i]) : 0u;
+        nan |= v[i] != v[i];
+    }
+    if (__any_sync(kFull, nan)) return false;
+#pragma unroll
+    for (int n = PER - 1; n > 0; --n)
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const bool swap = key[i] < key[i + 1];
+            const uint32_t k0 = swap ? key[i + 1] : key[i], k1 = swap ? key[i] : key[i + 1];
+            const int i0 = swap ? idx[i + 1] : idx[i], i1 = swap ? idx[i] : idx[i + 1];
+            key[i] = k0, key[i + 1] = k1, idx[i] = i0, idx[i + 1] = i1;
+        }
+    for (int j = 0; j < top_k; ++j) {
+        const uint32_t kmax = __reduce_max_sync(kFull, key[0]);
+        if (kmax <= kMinusInf) return false;
+        if (j == 0) row_max = key_float(kmax);
+        // one owner in all but tied rounds; redux is the slow instruction here, a vote and a shuffle are not
+        const unsigned owners = __ballot_sync(kFull, key[0] == kmax);
+        int e_win = __shfl_sync(kFull, idx[0], __ffs(owners) - 1);
+        if (owners & (owners - 1)) e_win = __reduce_min_sync(kFull, key[0] == kmax ? idx[0] : 0x7fffffff);
+        if (lane == j) {
+            my_val = key_float(kmax);
+            my_idx = e_win;
+        }
+        const bool mine = idx[0] == e_win;
+#pragma unroll
+        for (int i = 0; i + 1 < PER; ++i) {
+            key[i] = mine ? key[i + 1] : key[i];
+            idx[i] = mine ? idx[i + 1] : idx[i];
+        }
+        if (mine) key[PER - 1] = 0;
+    }
+    return true;
+}
+
 // PER = ceil(E / 32) rounded up to a power of two (1..32): registers per lane. On return lane j < top_k holds the
 // j-th selected expert (descending logit, ties to the lower index) and its routing weight.
-// Every lane caches the best of its own PER logits; a round is then two warp reductions (redux.sync: the largest
+// The general loop: every lane caches the best of its own PER logits; a round is then two warp reductions (redux.sync: the largest
 // key, and the lowest expert index among the lanes holding it) and only the winning lane rescans its registers.
 template <typename T, int PER>
 __device__ __forceinline__ void route_token_warp(const T *__restrict__ row, int E, int top_k, int renormalize, int lane,
@@ -41,6 +93,11 @@ __device__ __forceinline__ void route_token_warp(const T *__restrict__ row, int 
         const int e = lane + 32 * i;
         v[i] = e < E ? load_logit<T>(row + e) : -CUDART_INF_F;
     }
+    float m = 0.f, my_val = 0.f;
+    my_idx = 0;
+    const bool sorted = PER <= 8 && select_sorted<T, (PER <= 8 ? PER : 1)>(
+                                        *reinterpret_cast<const float(*)[PER <= 8 ? PER : 1]>(&v), E, top_k, lane, my_val,
+                                        my_idx, m);
     auto local_best = [&](uint32_t &key, int &best_e) {   // lowest index among this lane's largest logits
         float best = -CUDART_INF_F;
         best_e = 0x7fffffff;
@@ -56,8 +113,12 @@ __device__ __forceinline__ void route_token_warp(const T *__restrict__ row, int 
     };
     uint32_t lkey;
     int lbest;
-    local_best(lkey, lbest);
-    const float m = key_float(__reduce_max_sync(kFull, lkey));
+    if (!sorted) {
+        my_val = 0.f;
+        my_idx = 0;
+        local_best(lkey, lbest);
+        m = key_float(__reduce_max_sync(kFull, lkey));
+    }
     float sum = 0.f;
     if (!renormalize) {
 #pragma unroll
@@ -65,9 +126,7 @@ __device__ __forceinline__ void route_token_warp(const T *__restrict__ row, int 
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFull, sum, d);
     }
-    float my_val = 0.f;
-    my_idx = 0;
-    for (int j = 0; j < top_k; ++j) {
+    for (int j = 0; !sorted && j < top_k; ++j) {
         const uint32_t kmax = __reduce_max_sync(kFull, lkey);
         const int e_win = __reduce_min_sync(kFull, lkey == kmax ? lbest : 0x7fffffff);
         if (lane == j) {

@@ -198,3 +198,23 @@ def test_argument_checks():
     assert lib.pmoe_route_topk(lg.data_ptr(), 0, 4, 8, 9, 1, ids.data_ptr(), ids.data_ptr(), None) == 2   # top_k > E
     assert lib.pmoe_route_topk(lg.data_ptr(), 7, 4, 8, 2, 1, ids.data_ptr(), ids.data_ptr(), None) == 1   # dtype code
     assert lib.pmoe_route_topk(lg.data_ptr(), 0, 4, 2000, 2, 1, ids.data_ptr(), ids.data_ptr(), None) == 2
+
+
+@pytest.mark.parametrize("E,k", [(8, 2), (33, 5), (128, 8), (200, 8), (300, 8)])    # 1, 2, 4, 8 and 16 logits per lane
+def test_route_topk_ties_and_masked_logits(E, k):
+    """Ties resolve to the lower expert whatever lane holds it; rows with as many finite logits as top_k take exactly
+    those; the weights of a row do not depend on how its selection was made."""
+    import prime_flash_moe_b200 as P
+    g = torch.Generator().manual_seed(E)
+    logits = torch.randint(-3, 3, (64, E), generator=g).float()          # many ties
+    for t in range(32, 64):                                              # exactly k unmasked experts
+        keep = torch.randperm(E, generator=g)[:k]
+        row = torch.full((E,), float("-inf"))
+        row[keep] = logits[t, keep]
+        logits[t] = row
+    ids, wts = P.route_topk(logits.to(DEV), k)
+    for t in range(64):
+        order = sorted(range(E), key=lambda e: (-float(logits[t, e]), e))[:k]
+        assert ids[t].tolist() == order, t
+    ref = torch.softmax(torch.gather(logits, 1, ids.cpu().long()), -1)
+    torch.testing.assert_close(wts.cpu(), ref, rtol=1e-5, atol=1e-7)
