@@ -61,23 +61,28 @@ int set_error(int code, const char *fmt, ...) {
     return code;
 }
 
-int make_tmap_2d(CUtensorMap *map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void *base,
-                 uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols,
-                 CUtensorMapSwizzle swizzle, const char *what) {
+int make_tmap_nd(CUtensorMap *map, CUtensorMapDataType dtype, uint32_t rank, const void *base, const cuuint64_t *dims,
+                 const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle, const char *what) {
     auto encode = tensor_map_encoder();
     PMOE_REQUIRE(encode != nullptr, PMOE_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * elem_bytes};
-    const cuuint32_t box[2] = {box_cols, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(map, dtype, 2, const_cast<void *>(base), dims, strides, box, estr,
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = encode(map, dtype, rank, const_cast<void *>(base), dims, strides, box, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     PMOE_REQUIRE(r == CUDA_SUCCESS, PMOE_ERR_CUDA,
-                 "tensor map '%s' (rows %llu, cols %llu, box %ux%u) failed: CUresult %d", what,
-                 static_cast<unsigned long long>(rows), static_cast<unsigned long long>(cols), box_rows, box_cols,
+                 "tensor map '%s' (rank %u, extents %llu x %llu, box %ux%u) failed: CUresult %d", what, rank,
+                 static_cast<unsigned long long>(dims[1]), static_cast<unsigned long long>(dims[0]), box[1], box[0],
                  static_cast<int>(r));
     return PMOE_OK;
+}
+
+int make_tmap_2d(CUtensorMap *map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void *base,
+                 uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols,
+                 CUtensorMapSwizzle swizzle, const char *what) {
+    const cuuint64_t dims[2] = {cols, rows};
+    const cuuint64_t strides[1] = {cols * elem_bytes};
+    const cuuint32_t box[2] = {box_cols, box_rows};
+    return make_tmap_nd(map, dtype, 2, base, dims, strides, box, swizzle, what);
 }
 
 int sm_count() {
@@ -169,6 +174,19 @@ int short_boxes_mode() {
     return e ? atoi(e) & 3 : 3;
 }
 
+bool token_n_enabled() {   // read on every call
+    if (const char *e = getenv("PMOE_TOKN")) return e[0] != '0';
+    for (const char *name : {"PMOE_AGATHER", "PMOE_PREGATHER", "PMOE_DUAL", "PMOE_DOWN_BULK", "PMOE_PAIR_TAILS",
+                             "PMOE_SHORT_A"})
+        if (getenv(name)) return false;
+    return true;
+}
+
+bool token_n_forced() {
+    const char *e = getenv("PMOE_TOKN");
+    return e && e[0] == '1';
+}
+
 static int g_phase_mask = 7;
 int phase_mask() { return g_phase_mask; }
 
@@ -181,7 +199,9 @@ int status_fetch_bf16(int *value, bool reset);
 int status_fetch_mxfp8(int *value, bool reset);
 int status_fetch_ep(int *value, bool reset);
 int status_fetch_bwd(int *value, bool reset);
+int status_fetch_tokn(int *value, bool reset);
 int wait_ns_store_bwd(unsigned long long ns);
+int wait_ns_store_tokn(unsigned long long ns);
 int wait_ns_store_ep(unsigned long long ns);
 int wait_ns_store_bf16(unsigned long long ns);
 int wait_ns_store_mxfp8(unsigned long long ns);
@@ -217,13 +237,14 @@ extern "C" int pmoe_device_status(int *status) {
     using namespace pmoe;
     PMOE_REQUIRE(status != nullptr, PMOE_ERR_BAD_ARG, "pmoe_device_status: null pointer");
     PMOE_CUDA_OK(cudaDeviceSynchronize());
-    int a = 0, b = 0, c = 0, d = 0, e = 0;
+    int a = 0, b = 0, c = 0, d = 0, e = 0, f = 0;
     if (int rc = status_fetch_bf16(&a, false)) return rc;
+    if (int rc = status_fetch_tokn(&f, false)) return rc;
     if (int rc = status_fetch_bwd(&e, false)) return rc;
     if (int rc = status_fetch_mxfp8(&b, false)) return rc;
     if (int rc = status_fetch_misc(&c, false)) return rc;
     if (int rc = status_fetch_ep(&d, false)) return rc;
-    *status = a ? a : (b ? b : (c ? c : (d ? d : e)));
+    *status = a ? a : (f ? f : (b ? b : (c ? c : (d ? d : e))));
     if (*status) return set_error(PMOE_ERR_DEVICE, "a kernel gave up a bounded wait (device status %d)", *status);
     return PMOE_OK;
 }
@@ -232,6 +253,7 @@ extern "C" int pmoe_reset_device_status(void) {
     using namespace pmoe;
     PMOE_CUDA_OK(cudaDeviceSynchronize());
     if (int rc = status_fetch_bf16(nullptr, true)) return rc;
+    if (int rc = status_fetch_tokn(nullptr, true)) return rc;
     if (int rc = status_fetch_mxfp8(nullptr, true)) return rc;
     if (int rc = status_fetch_ep(nullptr, true)) return rc;
     if (int rc = status_fetch_bwd(nullptr, true)) return rc;
@@ -243,6 +265,7 @@ extern "C" int pmoe_debug_set_wait_ns(unsigned long long ns) {
     PMOE_REQUIRE(ns >= 1000ull && ns <= 60000000000ull, PMOE_ERR_BAD_ARG,
                  "pmoe_debug_set_wait_ns: the limit must lie between 1 microsecond and 60 seconds");
     if (int rc = wait_ns_store_bf16(ns)) return rc;
+    if (int rc = wait_ns_store_tokn(ns)) return rc;
     if (int rc = wait_ns_store_mxfp8(ns)) return rc;
     if (int rc = wait_ns_store_ep(ns)) return rc;
     if (int rc = wait_ns_store_bwd(ns)) return rc;

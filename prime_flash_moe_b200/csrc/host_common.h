@@ -32,6 +32,10 @@ int make_tmap_2d(CUtensorMap *map, CUtensorMapDataType dtype, uint32_t elem_byte
                  uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols,
                  CUtensorMapSwizzle swizzle, const char *what);
 
+// tensor map of any rank up to 5: extents, byte strides of dimensions 1.., box, innermost first
+int make_tmap_nd(CUtensorMap *map, CUtensorMapDataType dtype, uint32_t rank, const void *base, const cuuint64_t *dims,
+                 const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle, const char *what);
+
 // stream-ordered scratch from a private per-device pool (used by the entry points without `_ws`)
 int scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
 int scratch_free(void *ptr, cudaStream_t stream);
@@ -86,6 +90,12 @@ bool pair_tails_enabled();
 
 // PMOE_DUAL=0/1 forces one / two row blocks per tile in the one-CTA bf16 gate/up kernel; unset = -1 = by size
 int dual_blocks_mode();   // bit 0: loads, bit 1: activation stores
+
+// The bf16 split pipeline runs on the token-N kernels (moe_bf16_tokn.cu) where they are the faster ones, but not with
+// PMOE_TOKN=0, nor when one of the switches of the row-M kernels above is set (a caller who sets one means those
+// kernels); PMOE_TOKN=1 takes them at every size
+bool token_n_enabled();
+bool token_n_forced();
 
 // which launches of a split pipeline run (pmoe_debug_set_phase_mask): 1 gather, 2 gate/up, 4 down; 8 = without the
 // single-block tail launches of the bpc = 2 pipeline (to time the CTA-pair kernels alone)

@@ -40,6 +40,7 @@
 #include <algorithm>
 
 #include "host_common.h"
+#include "moe_bf16_tokn.h"
 #include "ptx.cuh"
 #include "tile_sched.cuh"
 
@@ -1536,10 +1537,11 @@ int set_smem(Kernel k, size_t bytes) {
 // Byte offsets of the regions a call may carve out of its workspace. ONE function answers both "how large must
 // the workspace be" and "where does the launcher put each region", whatever PMOE_PREGATHER / PMOE_AGATHER / bpc
 // select at call time: every region is always reserved.
-//   split != 0: activation [sorted_num, H] bf16 | x_sorted [sorted_num, K] bf16 | pair list, tail list, counts
+//   split != 0: activation [sorted_num, H] bf16 | x_sorted [sorted_num, K] bf16 | pair list, tail list, counts |
+//               work items of the token-N kernels
 //   split == 0: fp32 accumulation buffer [M, K] (padded to 1024 bytes) | x_sorted [sorted_num, K] bf16
 struct WorkspaceLayout {
-    size_t x_sorted, lists, total;
+    size_t x_sorted, lists, items, total;
 };
 WorkspaceLayout plan_workspace(int M, int K, int N, int sorted_num, int split) {
     WorkspaceLayout w{};
@@ -1553,7 +1555,8 @@ WorkspaceLayout plan_workspace(int M, int K, int N, int sorted_num, int split) {
     }
     w.x_sorted = rows * (N / 2) * 2;           // a multiple of 1024: sorted_num % 128 == 0 and H % 128 == 0
     w.lists = w.x_sorted + rows * K * 2;
-    w.total = up(w.lists + (rows / 128 + 8) * sizeof(int32_t));   // two lists of <= blocks/2 entries + two counts
+    w.items = up(w.lists + (rows / 128 + 8) * sizeof(int32_t));   // two lists of <= blocks/2 entries + two counts
+    w.total = up(w.items + tokn_items_bytes(static_cast<int>(rows)));
     return w;
 }
 
@@ -1563,6 +1566,7 @@ struct Decisions {
     int a_mode;       // gate/up A operand: 0 TMA gather4 from x, 1 row-gather pre-pass, 2 LSU gather in the kernel
     bool pregather;   // x_sorted region written and read
     bool tails;       // bpc == 2: pair / tail lists written and read
+    bool token_n;     // the token-N kernels run instead (x_sorted and the work items written and read)
 };
 Decisions decide(const Problem &p) {
     Decisions d{};
@@ -1576,6 +1580,19 @@ Decisions decide(const Problem &p) {
         d.a_mode = (p.bpc == 1 && p.N < 8192 && static_cast<long long>(p.M) * p.top_k >= 256ll * p.E) ? 2 : 1;
     d.pregather = d.a_mode == 1 || p.bpc == 2;   // the CTA-pair kernels always take pre-gathered rows
     d.tails = p.bpc == 2 && pair_tails_enabled();
+    // results addressed through out_rows may live in a peer's memory (plain vector reductions only) and kept
+    // pre-activations are stored per accumulator row: both stay with the row-M kernels
+    // ... and so do the narrowest layers: the row-gathered copy of x and the short down tiles cost the token-N kernels
+    // more than they gain there (row-M / token-N, us: N = 768, 949 rows per expert 187 / 228; N = 1024, 29 rows 152 / 168;
+    // N = 1024, 2813 rows 3160 / 4080; but N = 1536, 512 rows 801 / 724; N = 2048, 1911 rows 319 / 282; N = 3072, Zipf
+    // over 4096 rows 18090 / 16670)
+    // A batch whose gate/up tiles fill the SMs once but not the CTA pairs (each pair would take a second, mostly empty
+    // round) is left to the row-M kernels too when K is long (10 experts x 12 tiles, K = 3456: 67 / 70 us, but 18 x 8,
+    // K = 2176: 59 / 57; 5 x 25, K = 1408: 59 / 51).
+    const long long tiles = std::min<long long>(p.E, static_cast<long long>(p.M) * p.top_k) * (p.N / 256);
+    const bool second_round = 2 * tiles > sm_count() && tiles <= sm_count() && p.K >= 3072;
+    d.token_n = token_n_enabled() && !call_extras().out_rows && !call_extras().gu_out &&
+                ((p.N > 1024 && !second_round) || token_n_forced());
     return d;
 }
 
@@ -1678,9 +1695,14 @@ int run(const Problem &p, void *workspace, size_t workspace_bytes, cudaStream_t 
                  "fused_moe_bf16: workspace of %zu bytes required, got %zu", lay.total, workspace_bytes);
     uint8_t *const ws_base = static_cast<uint8_t *>(workspace);
     const Decisions dec = decide(p);
+    const int phases = phase_mask();  // profiling hook: 1 = gather, 2 = gate/up, 4 = down (default all)
+    if (dec.token_n) {
+        const ToknProblem t{p.x, p.w, p.w2, p.out, p.sorted_ids, p.expert_ids, p.npp, p.topk_weights, extras.live_rows,
+                            p.top_k, p.M, p.K, p.N, p.E, p.sorted_num, p.bpc};
+        return run_tokn_bf16(t, workspace, ws_base + lay.x_sorted, ws_base + lay.items, phases, stream);
+    }
     const int a_mode = dec.a_mode;
     const bool pregather = dec.pregather;
-    const int phases = phase_mask();  // profiling hook: 1 = gather, 2 = gate/up, 4 = down (default all)
     if (pregather) {
         __nv_bfloat16 *x_sorted = reinterpret_cast<__nv_bfloat16 *>(ws_base + lay.x_sorted);
         if (phases & 1) {
@@ -1925,6 +1947,7 @@ extern "C" size_t pmoe_debug_bf16_workspace_extent(int M, int K, int N, int num_
     size_t end = rows * (N / 2) * 2;                                  // activation
     if (d.pregather) end = std::max(end, lay.x_sorted + rows * K * 2);
     if (d.tails) end = std::max(end, lay.lists + (2 * (rows / 256) + 2) * sizeof(int32_t));
+    if (d.token_n) end = std::max(end, lay.items + tokn_items_bytes(sorted_num));
     return end;
 }
 

@@ -1,0 +1,775 @@
+// bf16 fused MoE FFN with the routed rows on the N side of the MMA ("token-N" kernels), sm_100a, CTA pairs.
+//
+// tcgen05 fixes M at 128 or 256 but takes any multiple of 16 as N. With the rows as M (moe_bf16.cu) an expert pays
+// for whole 128-row blocks: 8 rows of a decode batch cost a 128-row MMA, 530 rows cost 640. Here the WEIGHT rows are
+// M (256 per CTA pair, cta_group::2) and an expert's routed rows are N, cut into equal pieces of at most `cap` rows
+// (a multiple of 32): 530 rows run as 3 x 192, and the operand feed per CTA and k-step is 16 KB of weights + up to
+// 16 KB of rows instead of 48 KB for the same MACs of a one-CTA 128 x 256 tile.
+//
+//   work item   (expert, first row of sorted_token_ids, rows of this piece): built on the device by CTA 0 of
+//               gather_plan_kernel while the other CTAs copy the routed rows of x into x_sorted
+//   gate/up     tile = item x 128 activation columns. Each CTA of the pair owns 64 of them: its A tile holds the 64
+//               gate rows and the 64 up rows interleaved in groups of 16 (ONE five-dimensional TMA box per k-step), so
+//               that lanes l and l + 16 of a TMEM lane quarter hold gate and up of the same activation and two
+//               16-lane TMEM loads give a thread both. SwiGLU -> bf16 -> staging -> TMA store.
+//   down        tile = item x 256 output columns, 128 per CTA; accumulator * routing weight -> bf16 -> staging rows
+//               (one per routed row) -> one 256-byte bulk reduction into out[token] each (plain 16-byte vector
+//               reductions by the store warp, two rows per instruction, were 8 % slower at H = 768).
+//
+// Warp roles: warp 0 TMA producer, warp 1 TMEM owner + MMA issuer (even CTA), warps 2-9 epilogue in two groups of four
+// (a group takes every second 32-row chunk of the accumulator), warps 10-11 one store warp per group: it waits for a
+// staged chunk, issues the bulk stores and hands the buffer back, so that the epilogue warps never wait for a store
+// to be read. Two 256-column accumulators in TMEM; every wait is bounded (ptx.cuh).
+#include <algorithm>
+#include <atomic>
+
+#include "host_common.h"
+#include "moe_bf16_tokn.h"
+#include "ptx.cuh"
+#include "tile_sched.cuh"
+
+namespace pmoe {
+
+__device__ int g_status_tokn = 0;
+
+namespace {
+
+constexpr int BM = kBlockM;
+constexpr int BK = 64;
+constexpr uint32_t A_BYTES = 128 * BK * 2;       // 16 KB: 128 weight rows per CTA and k-step
+constexpr int MAX_STAGES = 12;
+constexpr uint32_t TMEM_COLS = 512;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = (2 + EPI_WARPS + 2) * 32;
+constexpr int CHUNK = 32;                        // rows per staged chunk
+constexpr int UP_BUFS = 4, DOWN_BUFS = 3;        // staging buffers per epilogue group
+constexpr uint32_t UP_BUF_BYTES = CHUNK * 128;           // 32 rows x 64 activation columns, 128-byte swizzle
+constexpr uint32_t DOWN_ROW_BYTES = 256 + 16;            // 128 output columns, padded against bank conflicts
+constexpr uint32_t DOWN_BUF_BYTES = CHUNK * DOWN_ROW_BYTES;
+constexpr uint32_t UP_STAGING = 2 * UP_BUFS * UP_BUF_BYTES;       // 32 KB
+constexpr uint32_t DOWN_STAGING = 2 * DOWN_BUFS * DOWN_BUF_BYTES; // 51 KB
+constexpr uint32_t BAR_BYTES = 512;
+constexpr uint32_t SMEM_LIMIT = 232448;
+constexpr int ST_BAD_PAIR = 8;                   // bpc = 2 table whose 256-row pair holds two experts
+
+struct Args {
+    const int2 *row_info;     // per sorted row: token (-1 for padding) and routing weight (fp32 bits)
+    __nv_bfloat16 *out;
+    const int32_t *live_rows;
+    const int4 *items;        // end of the item buffer: item i of n is items[i - n] (the planner fills it backwards)
+    const int32_t *item_count;
+    int M, K, H;
+    int stages;
+    uint32_t stage_bytes;
+    int use_pdl, zero_out;
+};
+
+struct Smem {
+    uint32_t ring, staging, bars, stage_bytes;
+    __device__ __forceinline__ uint32_t a(int s) const { return ring + s * stage_bytes; }
+    __device__ __forceinline__ uint32_t b(int s) const { return ring + s * stage_bytes + A_BYTES; }
+    __device__ __forceinline__ uint32_t full(int s) const { return bars + 8 * s; }
+    __device__ __forceinline__ uint32_t empty(int s) const { return bars + 8 * (MAX_STAGES + s); }
+    __device__ __forceinline__ uint32_t tmem_full(int b) const { return bars + 8 * (2 * MAX_STAGES + b); }
+    __device__ __forceinline__ uint32_t tmem_empty(int b) const { return bars + 8 * (2 * MAX_STAGES + 2 + b); }
+    __device__ __forceinline__ uint32_t staged(int i) const { return bars + 8 * (2 * MAX_STAGES + 4 + i); }
+    __device__ __forceinline__ uint32_t freed(int i) const { return bars + 8 * (2 * MAX_STAGES + 4 + 2 * UP_BUFS + i); }
+    __device__ __forceinline__ uint32_t tmem_slot() const { return bars + 8 * (2 * MAX_STAGES + 4 + 4 * UP_BUFS); }
+};
+
+size_t smem_bytes(int stages, uint32_t stage_bytes, bool up) {
+    return 1024 + static_cast<size_t>(stages) * stage_bytes + (up ? UP_STAGING : DOWN_STAGING) + BAR_BYTES;
+}
+
+__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar_cluster_addr, int c0,
+                                                 int c1, int c2, int c3, int c4) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+        : "memory");
+}
+// 16 lanes x 32 columns of 32-bit in the fragment layout of an m16n8 accumulator: with i = lane id, d[4 j + {0, 1}] are
+// columns 8 j + 2 (i % 4) + {0, 1} of TMEM lane i / 4, d[4 j + {2, 3}] the same columns of lane i / 4 + 8
+__device__ __forceinline__ void tmem_ld_16x256b_x4(float (&d)[16], uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]), "=f"(d[4]), "=f"(d[5]), "=f"(d[6]), "=f"(d[7]), "=f"(d[8]),
+          "=f"(d[9]), "=f"(d[10]), "=f"(d[11]), "=f"(d[12]), "=f"(d[13]), "=f"(d[14]), "=f"(d[15])
+        : "r"(addr)
+        : "memory");
+}
+// four 8 x 8 matrices of bf16 fragments stored transposed; lane i gives the address of row i % 8 of matrix i / 8
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b),
+                 "r"(c), "r"(d)
+                 : "memory");
+}
+
+// whole warp waits through lane 0
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int *status, int code, int lane) {
+    bool ok = true;
+    if (lane == 0) ok = mbar_wait(bar, parity, status, code);
+    return __shfl_sync(0xffffffffu, ok, 0);
+}
+
+// ---------------------------------------------------------------------------------------------
+// work items (CTA 0 of gather_plan_kernel). A run is a maximal sequence of consecutive row blocks of one expert whose
+// blocks, except the last, are full; its n rows are cut into ceil(n / cap) pieces of equal size rounded up to 32 rows.
+// Runs are found from the end of the table to its start, 512 blocks at a time, so that a run's first block already
+// knows where the run ends; the items are written backwards from `items_end`, in table order.
+// ---------------------------------------------------------------------------------------------
+constexpr int PLAN_THREADS = 512;
+
+// ext[i] = rows of block c0 + i up to and including the last routed one, for the chunk's 512 blocks; a warp reads a block
+// with one load, eight blocks in flight
+__device__ __forceinline__ void block_extents(const int32_t *sorted_ids, int c0, int blocks, int *ext) {
+    constexpr int kWarps = PLAN_THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int u0 = 0; u0 < 32 && c0 + u0 * kWarps < blocks; u0 += 8) {
+        int4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int b = c0 + (u0 + u) * kWarps + warp;
+            v[u] = make_int4(-1, -1, -1, -1);
+            if (b < blocks) v[u] = reinterpret_cast<const int4 *>(sorted_ids + static_cast<size_t>(b) * BM)[lane];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int last = v[u].w >= 0 ? 3 : v[u].z >= 0 ? 2 : v[u].y >= 0 ? 1 : v[u].x >= 0 ? 0 : -1;
+            const int rows = __reduce_max_sync(0xffffffffu, last >= 0 ? 4 * lane + last + 1 : 0);
+            if (lane == 0) ext[(u0 + u) * kWarps + warp] = rows;
+        }
+    }
+}
+
+__device__ void plan_items(const int32_t *__restrict__ sorted_ids, const int32_t *__restrict__ expert_ids, int blocks,
+                           int cap, int bpc, int4 *items_end, int32_t *item_count) {
+    constexpr int kWarps = PLAN_THREADS / 32;
+    __shared__ int s_first[kWarps];    // first run start of every warp's 32 blocks (or INT_MAX)
+    __shared__ int s_sum[kWarps];
+    __shared__ int s_ext[PLAN_THREADS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int next_chunk = blocks;   // first run start after this chunk ...
+    int next_ext = 0;          // ... and the extent of the block before it
+    int written = 0;           // items of the later chunks
+    for (int c0 = (blocks - 1) / PLAN_THREADS * PLAN_THREADS; c0 >= 0; c0 -= PLAN_THREADS) {
+        const int b = c0 + threadIdx.x;
+        block_extents(sorted_ids, c0, blocks, s_ext);
+        bool start = false;
+        int e = 0;
+        if (b < blocks) {
+            e = expert_ids[b];
+            start = b == 0 || expert_ids[b - 1] != e || sorted_ids[static_cast<size_t>(b) * BM - 1] < 0;
+            if (bpc == 2 && (b & 1) && expert_ids[b - 1] != e) atomicCAS(&g_status_tokn, 0, ST_BAD_PAIR);
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, start);
+        if (lane == 0) s_first[warp] = m ? c0 + warp * 32 + __ffs(m) - 1 : 0x7fffffff;
+        __syncthreads();
+        int next = next_chunk, first = next_chunk;
+        for (int w = kWarps - 1; w >= 0; --w) {
+            const int f = s_first[w];
+            if (f != 0x7fffffff) {
+                first = f;
+                if (w > warp) next = f;
+            }
+        }
+        const uint32_t later = lane < 31 ? m >> (lane + 1) : 0u;
+        if (later) next = b + __ffs(later);
+        int n = 0, pieces = 0;
+        if (start) {
+            const int last = next - 1;
+            n = (last - b) * BM + (last < c0 + PLAN_THREADS ? s_ext[last - c0] : next_ext);
+            pieces = (n + cap - 1) / cap;
+        }
+        int suffix = pieces;      // items of this and the later blocks of the chunk
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_down_sync(0xffffffffu, suffix, d);
+            if (lane + d < 32) suffix += v;
+        }
+        if (lane == 0) s_sum[warp] = suffix;
+        __syncthreads();
+        int total = 0;
+        for (int w = 0; w < kWarps; ++w) {
+            const int v = s_sum[w];
+            total += v;
+            if (w > warp) suffix += v;
+        }
+        if (pieces) {
+            const int width = ((n + pieces - 1) / pieces + 31) & ~31;
+            int4 *dst = items_end - written - suffix;
+            for (int i = 0; i < pieces; ++i) {
+                const int r0 = i * width;
+                const int rows = min(width, ((n - r0) + 31) & ~31);
+                dst[i] = make_int4(e, b * BM + r0, max(rows, 0), 0);
+            }
+        }
+        written += total;
+        // a run of an earlier chunk that reaches into this one ends before this one's first run start, or at the end
+        if (first < next_chunk) {
+            if (first > c0) next_ext = s_ext[first - 1 - c0];
+        } else if (blocks > c0 && blocks <= c0 + PLAN_THREADS) {
+            next_ext = s_ext[blocks - 1 - c0];
+        }
+        next_chunk = first;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *item_count = written;
+}
+
+// CTA 0 builds the work items; the other CTAs copy x_sorted[row] = x[token(row)], one warp per row (padding rows are
+// left as they are: they feed accumulator columns that nothing reads), and write the row's token and routing weight
+// where the down kernel finds both with one load instead of two dependent ones.
+__global__ void __launch_bounds__(PLAN_THREADS)
+gather_plan_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ x_sorted,
+                   const int32_t *__restrict__ sorted_ids, const int32_t *__restrict__ expert_ids,
+                   const int32_t *__restrict__ npp, const float *__restrict__ topk_weights, int M, int K, int top_k,
+                   int sorted_num, int cap, int bpc, int4 *items_end, int32_t *item_count, int2 *__restrict__ row_info) {
+    pdl_wait_primary();        // launched as a programmatic dependent of whatever the stream holds: the routing kernel
+    pdl_launch_dependents();
+    const int blocks = live_row_blocks(npp, sorted_num);
+    if (blockIdx.x == 0) {
+        plan_items(sorted_ids, expert_ids, blocks, cap, bpc, items_end, item_count);
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const int rows = blocks * BM;
+    const int chunks = K / 8;
+    constexpr int kWarps = PLAN_THREADS / 32;
+    for (int row = (blockIdx.x - 1) * kWarps + (threadIdx.x >> 5); row < rows; row += (gridDim.x - 1) * kWarps) {
+        const int pair = sorted_ids[row];
+        const int tok = pair >= 0 ? pair / top_k : -1;
+        const bool live = tok >= 0 && tok < M;
+        if (lane == 0) row_info[row] = make_int2(live ? tok : -1, live ? __float_as_int(topk_weights[pair]) : 0);
+        if (!live) continue;
+        const int4 *src = reinterpret_cast<const int4 *>(x + static_cast<size_t>(tok) * K);
+        int4 *dst = reinterpret_cast<int4 *>(x_sorted + static_cast<size_t>(row) * K);
+#pragma unroll 4
+        for (int ch = lane; ch < chunks; ch += 32) dst[ch] = __ldg(src + ch);
+    }
+}
+
+// The same preparation in two launches for activations that do not stay in L2: the row info with its inverse (sorted row
+// of every routed pair), then, beside the work items, x read token by token - once instead of top_k times - and written to
+// the token's rows. T = 65536, K = 4096, top_k = 8: 8.6 GB of traffic in 1.45 ms one way, 4.8 GB in 0.9 ms this way; with
+// x in L2 (T = 8192, K = 2048: 64 us) only the writes count.
+__global__ void __launch_bounds__(PLAN_THREADS)
+row_info_kernel(const int32_t *__restrict__ sorted_ids, const int32_t *__restrict__ npp,
+                const float *__restrict__ topk_weights, int M, int top_k, int sorted_num, int2 *__restrict__ row_info,
+                int32_t *__restrict__ inv) {
+    pdl_wait_primary();
+    pdl_launch_dependents();
+    const int rows = live_row_blocks(npp, sorted_num) * BM;
+    for (int row = blockIdx.x * PLAN_THREADS + threadIdx.x; row < rows; row += gridDim.x * PLAN_THREADS) {
+        const int pair = sorted_ids[row];
+        const int tok = pair >= 0 ? pair / top_k : -1;
+        const bool live = tok >= 0 && tok < M;
+        row_info[row] = make_int2(live ? tok : -1, live ? __float_as_int(topk_weights[pair]) : 0);
+        if (live) inv[pair] = row;
+    }
+}
+
+// CTA 0 builds the work items; in the others one warp per token. inv is not initialised: an entry counts only if the row it names holds that very pair (pairs that
+// the routing table leaves out have no row).
+__global__ void __launch_bounds__(PLAN_THREADS)
+gather_tokens_plan_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ x_sorted,
+                          const int32_t *__restrict__ sorted_ids, const int32_t *__restrict__ expert_ids,
+                          const int32_t *__restrict__ npp, const int32_t *__restrict__ inv, int M, int K, int top_k,
+                          int sorted_num, int cap, int bpc, int4 *items_end, int32_t *item_count) {
+    pdl_wait_primary();
+    pdl_launch_dependents();
+    const int blocks = live_row_blocks(npp, sorted_num);
+    if (blockIdx.x == 0) {
+        plan_items(sorted_ids, expert_ids, blocks, cap, bpc, items_end, item_count);
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const int rows = blocks * BM;
+    const int chunks = K / 8;
+    constexpr int kWarps = PLAN_THREADS / 32;
+    for (int t = (blockIdx.x - 1) * kWarps + (threadIdx.x >> 5); t < M; t += (gridDim.x - 1) * kWarps) {
+        int row = -1;
+        if (lane < top_k) {
+            const int pair = t * top_k + lane;
+            const int r = inv[pair];
+            if (r >= 0 && r < rows && sorted_ids[r] == pair) row = r;
+        }
+        const uint32_t routed = __ballot_sync(0xffffffffu, row >= 0);
+        if (routed == 0) continue;
+        const int4 *src = reinterpret_cast<const int4 *>(x + static_cast<size_t>(t) * K);
+        for (int c0 = 0; c0 < chunks; c0 += 8 * 32) {
+            int4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int c = c0 + i * 32 + lane;
+                if (c < chunks) v[i] = __ldg(src + c);
+            }
+            for (uint32_t m = routed; m; m &= m - 1) {
+                int4 *dst = reinterpret_cast<int4 *>(x_sorted + static_cast<size_t>(__shfl_sync(0xffffffffu, row, __ffs(m) - 1)) * K);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int c = c0 + i * 32 + lane;
+                    if (c < chunks) dst[c] = v[i];
+                }
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// the GEMM kernel
+// ---------------------------------------------------------------------------------------------
+struct Tile {
+    int expert, row0, rows, n_tile;
+};
+// Every role fetches the tile after the one it works on: the item comes from L2 (0.4 us), a tenth of a short tile.
+__device__ __forceinline__ Tile fetch_tile(const int4 *items, int t, int num_tiles, int n_items, int n_tiles) {
+    Tile w{0, 0, 0, 0};
+    if (t < num_tiles) {
+        const Coord c = tile_coord(t, n_items, n_tiles);
+        const int4 it = items[c.m_blk];
+        w.expert = it.x, w.row0 = it.y, w.rows = it.z, w.n_tile = c.n_tile;
+    }
+    return w;
+}
+// token / weight of the rows `lane` of an epilogue group's (at most four) chunks
+__device__ __forceinline__ void fetch_rows(const int2 *row_info, const Tile &w, int grp, int lane, int2 (&r)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int ch = grp + 2 * j;
+        r[j] = make_int2(-1, 0);
+        if (ch * CHUNK < w.rows) r[j] = row_info[w.row0 + ch * CHUNK + lane];
+    }
+}
+
+template <bool kUp>
+__global__ void __launch_bounds__(THREADS, 1)
+moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_rows64,
+                const __grid_constant__ CUtensorMap map_rows16, const __grid_constant__ CUtensorMap map_act,
+                const Args a) {
+    extern __shared__ uint8_t smem_raw[];
+    constexpr int kBufs = kUp ? UP_BUFS : DOWN_BUFS;
+    constexpr uint32_t kBufBytes = kUp ? UP_BUF_BYTES : DOWN_BUF_BYTES;
+    Smem sm;
+    sm.stage_bytes = a.stage_bytes;
+    sm.ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    sm.staging = sm.ring + a.stages * a.stage_bytes;
+    sm.bars = sm.staging + 2 * kBufs * kBufBytes;
+    int *status = &g_status_tokn;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const bool leader = rank == 0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < a.stages; ++s) {
+            mbar_init(sm.full(s), 1);
+            mbar_init(sm.empty(s), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(sm.tmem_full(b), 1);
+            mbar_init(sm.tmem_empty(b), 2 * EPI_WARPS);
+        }
+        for (int i = 0; i < 2 * kBufs; ++i) {
+            mbar_init(sm.staged(i), 4);
+            mbar_init(sm.freed(i), 1);
+        }
+        fence_mbar_init();
+        tma_prefetch_desc(&map_w);
+        tma_prefetch_desc(&map_rows64);
+        tma_prefetch_desc(&map_rows16);
+        if (kUp) tma_prefetch_desc(&map_act);
+    }
+    if (warp == 1) tmem_alloc_pair(sm.tmem_slot(), TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();      // both CTAs' barriers are initialised and both halves of TMEM allocated
+    tc_fence_after();
+    uint32_t tmem_base;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(sm.tmem_slot()));
+
+    // a dependent CTA that shares this SM then blocks in its own TMEM allocation until this CTA has freed its columns
+    if (kUp) pdl_launch_dependents();
+    if (a.use_pdl) pdl_wait_primary();
+
+    const int n_items = *a.item_count;
+    const int4 *items = a.items - n_items;
+    const int n_tiles = kUp ? a.H / 128 : (a.K + 255) / 256;
+    const int num_tiles = n_items * n_tiles;
+    const int ksteps = (kUp ? a.K : a.H) / BK;
+    const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    auto fetch = [&](int t) { return fetch_tile(items, t, num_tiles, n_items, n_tiles); };
+
+    if (warp == 0) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t ph = 0;
+            long long issued = 0;
+            bool ok = true;
+            Tile w, next = fetch(first);
+            for (int t = first; t < num_tiles && ok; t += step) {
+                w = next;
+                next = fetch(t + step);
+                const int half = w.rows >> 1;
+                const int row0 = w.row0 + static_cast<int>(rank) * half;
+                const bool big = half > 32;
+                const int box = big ? 64 : 16;
+                const int boxes = (half + box - 1) / box;
+                const uint32_t bytes = 2 * (A_BYTES + static_cast<uint32_t>(boxes * box) * 128u);
+                for (int ks = 0; ks < ksteps; ++ks) {
+                    ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
+                    if (!ok) break;
+                    const uint32_t full_leader = mapa_shared(sm.full(s), 0);
+                    if (leader) mbar_arrive_expect_tx(sm.full(s), bytes);
+                    if (kUp)
+                        tma_load_5d_pair(sm.a(s), &map_w, full_leader, ks * BK, 0, 0,
+                                         w.n_tile * 8 + static_cast<int>(rank) * 4, w.expert);
+                    else
+                        tma_load_2d_pair(sm.a(s), &map_w, full_leader, ks * BK,
+                                         w.expert * a.K + w.n_tile * 256 + static_cast<int>(rank) * 128);
+                    for (int j = 0; j < boxes; ++j)
+                        tma_load_2d_pair(sm.b(s) + j * box * 128, big ? &map_rows64 : &map_rows16, full_leader, ks * BK,
+                                         row0 + j * box);
+                    ++issued;
+                    if (++s == a.stages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+            if (!ok && leader) {
+                // give the copies already issued (both CTAs' bytes arrive here) a bounded time to land
+                const long long f0 = issued > a.stages ? issued - a.stages : 0;
+                for (long long f = f0; f < issued; ++f) {
+                    const uint32_t bar = sm.full(static_cast<int>(f % a.stages));
+                    const uint32_t parity = static_cast<uint32_t>((f / a.stages) & 1);
+                    const uint64_t t0 = globaltimer_ns();
+                    while (!mbar_try_wait(bar, parity))
+                        if (globaltimer_ns() - t0 > 20000000ull) break;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (leader && elect_one()) {
+            int s = 0;
+            uint32_t ph = 0;
+            int it_n = 0;
+            bool ok = true;
+            Tile w, next = fetch(first);
+            for (int t = first; t < num_tiles && ok; t += step, ++it_n) {
+                w = next;
+                next = fetch(t + step);
+                const uint32_t idesc = idesc_bf16_f32(256, static_cast<uint32_t>(w.rows));
+                const int buf = it_n & 1;
+                ok = mbar_wait_cluster(sm.tmem_empty(buf), ((it_n >> 1) & 1) ^ 1, status, ST_TIMEOUT_TMEM_EMPTY);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d = tmem_base + buf * 256;
+                for (int ks = 0; ks < ksteps; ++ks) {
+                    ok = mbar_wait(sm.full(s), ph, status, ST_TIMEOUT_FULL);
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k)
+                        umma_f16_pair(d, smem_desc_sw128(sm.a(s) + k * 32), smem_desc_sw128(sm.b(s) + k * 32), idesc,
+                                      (ks | k) != 0);
+                    umma_commit_pair(sm.empty(s), 3);
+                    if (++s == a.stages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (ok) umma_commit_pair(sm.tmem_full(buf), 3);
+            }
+        }
+        __syncwarp();
+    } else if (warp < 2 + EPI_WARPS) {
+        // ---------------- epilogue ----------------
+        const int grp = (warp - 2) >> 2;
+        const uint32_t quarter = warp & 3;
+        const uint32_t lane_base = quarter * 32;
+        if (kUp && a.zero_out) {
+            int4 *o4 = reinterpret_cast<int4 *>(a.out);
+            const long long live = a.live_rows ? max(0, min(a.M, *a.live_rows)) : a.M;
+            const long long n4 = live * a.K / 8;
+            const int4 z = make_int4(0, 0, 0, 0);
+            for (long long i = static_cast<long long>(blockIdx.x) * (EPI_WARPS * 32) + (threadIdx.x - 64); i < n4;
+                 i += static_cast<long long>(gridDim.x) * (EPI_WARPS * 32))
+                o4[i] = z;
+        }
+        // Lanes are weight rows, columns routed rows: the accumulator has to be transposed on its way to the staging
+        // buffer. The 16-lane TMEM load gives matrix fragments that stmatrix stores transposed, eight elements a lane.
+        // (One column a thread and 2-byte stores with a shuffle per element was bound by them: 4 us a tile.)
+        const uint32_t mat = lane >> 3, mrow = lane & 7;
+        const uint32_t off = kUp ? (8 * (mat >> 1) + mrow) * 128 + (((2 * quarter + (mat & 1)) ^ mrow) << 4)
+                                 : mrow * DOWN_ROW_BYTES + (quarter * 32 + 8 * mat) * 2;
+        int it_n = 0;
+        uint32_t chunk_n = 0;       // chunks of this group so far
+        bool ok = true;
+        Tile w, next = fetch(first);
+        int2 info[4], info_next[4];
+        if (!kUp) fetch_rows(a.row_info, next, grp, lane, info_next);
+        for (int t = first; t < num_tiles && ok; t += step, ++it_n) {
+            w = next;
+            next = fetch(t + step);
+            const int chunks = w.rows / CHUNK;
+            const int buf = it_n & 1;
+            if (!kUp) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) info[j] = info_next[j];
+            }
+            ok = warp_wait(sm.tmem_full(buf), (it_n >> 1) & 1, status, ST_TIMEOUT_TMEM_FULL, lane);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t acc = tmem_base + buf * 256;
+            if (!kUp) fetch_rows(a.row_info, next, grp, lane, info_next);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int ch = grp + 2 * j;
+                if (ch >= chunks) break;
+                float lo[16], hi[16];      // up: 16 gate rows, 16 up rows; down: output columns 0-15, 16-31 of the quarter
+                tmem_ld_16x256b_x4(lo, tmem_addr(acc, lane_base, ch * CHUNK));
+                tmem_ld_16x256b_x4(hi, tmem_addr(acc, lane_base + 16, ch * CHUNK));
+                const uint32_t slot = chunk_n % kBufs, round = chunk_n / kBufs;
+                const uint32_t base = sm.staging + (grp * kBufs + slot) * kBufBytes + off;
+                ok = warp_wait(sm.freed(grp * kBufs + slot), (round & 1) ^ 1, status, ST_TIMEOUT_ACT, lane);
+                tmem_ld_wait();
+                if (!ok) break;
+                if (kUp) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) lo[i] = swiglu(lo[i], hi[i]);
+#pragma unroll
+                    for (int p = 0; p < 2; ++p)     // 16 routed rows x 16 activations
+                        stmatrix_x4_trans(base + p * 16 * 128, pack_bf16x2(lo[8 * p], lo[8 * p + 1]),
+                                          pack_bf16x2(lo[8 * p + 2], lo[8 * p + 3]), pack_bf16x2(lo[8 * p + 4], lo[8 * p + 5]),
+                                          pack_bf16x2(lo[8 * p + 6], lo[8 * p + 7]));
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {   // 8 routed rows x 32 output columns
+                        const int r = 8 * q + 2 * (lane & 3);
+                        const float w0 = __int_as_float(__shfl_sync(0xffffffffu, info[j].y, r));
+                        const float w1 = __int_as_float(__shfl_sync(0xffffffffu, info[j].y, r + 1));
+                        stmatrix_x4_trans(base + q * 8 * DOWN_ROW_BYTES, pack_bf16x2(w0 * lo[4 * q], w1 * lo[4 * q + 1]),
+                                          pack_bf16x2(w0 * lo[4 * q + 2], w1 * lo[4 * q + 3]),
+                                          pack_bf16x2(w0 * hi[4 * q], w1 * hi[4 * q + 1]),
+                                          pack_bf16x2(w0 * hi[4 * q + 2], w1 * hi[4 * q + 3]));
+                    }
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sm.staged(grp * kBufs + slot));
+                ++chunk_n;
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa_shared(sm.tmem_empty(buf), 0));
+        }
+    } else {
+        // ---------------- store warps ----------------
+        const int grp = warp - 2 - EPI_WARPS;
+        uint32_t chunk_n = 0;
+        bool ok = true;
+        Tile w, next = fetch(first);
+        int2 info[4], info_next[4];
+        if (!kUp) fetch_rows(a.row_info, next, grp, lane, info_next);
+        for (int t = first; t < num_tiles && ok; t += step) {
+            w = next;
+            next = fetch(t + step);
+            const int chunks = w.rows / CHUNK;
+            const int col0 = kUp ? w.n_tile * 128 + static_cast<int>(rank) * 64
+                                 : w.n_tile * 256 + static_cast<int>(rank) * 128;
+            if (!kUp) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) info[j] = info_next[j];
+                fetch_rows(a.row_info, next, grp, lane, info_next);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int ch = grp + 2 * j;
+                if (ch >= chunks) break;
+                const uint32_t slot = chunk_n % kBufs, round = chunk_n / kBufs;
+                const uint32_t base = sm.staging + (grp * kBufs + slot) * kBufBytes;
+                ok = warp_wait(sm.staged(grp * kBufs + slot), round & 1, status, ST_TIMEOUT_ACT, lane);
+                if (!ok) break;
+                if (kUp) {
+                    if (lane == 0) tma_store_2d(&map_act, base, col0, w.row0 + ch * CHUNK);
+                } else if (info[j].x >= 0 && col0 < a.K) {
+                    bulk_reduce_add_bf16(a.out + static_cast<size_t>(info[j].x) * a.K + col0, base + lane * DOWN_ROW_BYTES,
+                                         256);
+                }
+                tma_store_commit();
+                tma_store_wait_read<1>();      // the previous chunk's buffer has been read
+                __syncwarp();
+                if (chunk_n > 0 && lane == 0) mbar_arrive(sm.freed(grp * kBufs + (chunk_n - 1) % kBufs));
+                ++chunk_n;
+            }
+        }
+        tma_store_wait<0>();
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();      // nobody frees TMEM or exits while the peer may still use this CTA's memory
+    if (warp == 1) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+}
+
+// w1 [E, 2H, K] as (K, 16, gate | up, H / 16, E): one box = 64 k x (16 gate rows, 16 up rows) x 4 groups
+int make_gate_up_map(CUtensorMap *map, const void *w, int E, int H, int K) {
+    const cuuint64_t k2 = static_cast<cuuint64_t>(K) * 2;
+    const cuuint64_t dims[5] = {static_cast<cuuint64_t>(K), 16, 2, static_cast<cuuint64_t>(H) / 16,
+                                static_cast<cuuint64_t>(E)};
+    const cuuint64_t strides[4] = {k2, static_cast<cuuint64_t>(H) * k2, 16 * k2, 2 * static_cast<cuuint64_t>(H) * k2};
+    const cuuint32_t box[5] = {64, 16, 2, 4, 1};
+    return make_tmap_nd(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                        "w (gate | up interleaved)");
+}
+
+template <bool kUp>
+int launch(const CUtensorMap &mw, const CUtensorMap &m64, const CUtensorMap &m16, const CUtensorMap &mact, Args a,
+           uint32_t stage_bytes, long long max_tiles, cudaStream_t stream) {
+    a.stage_bytes = stage_bytes;
+    const uint32_t fixed = 1024 + (kUp ? UP_STAGING : DOWN_STAGING) + BAR_BYTES;
+    a.stages = std::min<int>(MAX_STAGES, static_cast<int>((SMEM_LIMIT - fixed) / stage_bytes));
+    const size_t smem = smem_bytes(a.stages, stage_bytes, kUp);
+    auto kernel = moe_tokn_kernel<kUp>;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.use_pdl ? 2 : 1;
+    // CTA pairs that fit the device: one a SM pair whatever the ring depth, asked for once per device
+    static std::atomic<int> pairs_of[64];
+    int dev = 0;
+    PMOE_CUDA_OK(cudaGetDevice(&dev));
+    PMOE_REQUIRE(dev >= 0 && dev < 64, PMOE_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+    int max_clusters = pairs_of[dev].load(std::memory_order_acquire);
+    if (max_clusters == 0) {
+        PMOE_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMEM_LIMIT)));
+        cudaLaunchConfig_t probe = cfg;
+        probe.gridDim = dim3(2);
+        probe.numAttrs = 1;
+        PMOE_CUDA_OK(cudaOccupancyMaxActiveClusters(&max_clusters, kernel, &probe));
+        if (max_clusters < 1) return set_error(PMOE_ERR_CUDA, "no CTA pair of the token-N kernel fits on this device");
+        pairs_of[dev].store(max_clusters, std::memory_order_release);
+    }
+    cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<long long>(max_tiles, max_clusters)));
+    PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, mw, m64, m16, mact, a));
+    return PMOE_OK;
+}
+
+}  // namespace
+
+// Rows of one work item at most, from the average rows per expert. Weight streaming wants many small ring slots (nine
+// of 20 KB at cap 64), compute wants wide accumulators (256 leaves TMEM for a second one); a cap below an expert's rows
+// reads its weights once per piece. Measured, us at cap 64 / 128 / 256: 28 rows 270 / 272 / 282; 41 rows 236 / 218 /
+// 221; 65 rows 423 / 359 / 377; 122 rows 188 / 148 / 149; 140 rows 1118 / 862 / 777.
+static int tokn_cap(const ToknProblem &p) {
+    const long long rows = static_cast<long long>(p.M) * p.top_k;
+    return rows <= 32ll * p.E ? 64 : rows <= 112ll * p.E ? 128 : 256;
+}
+
+// the count, at most two pieces per 128-row block (cap 64), the row info and its inverse
+size_t tokn_items_bytes(int sorted_num) {
+    return (static_cast<size_t>(sorted_num / BM) * 2 + 1) * sizeof(int4) +
+           static_cast<size_t>(sorted_num) * (sizeof(int2) + sizeof(int32_t));
+}
+
+int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, int phases, cudaStream_t stream) {
+    const int H = p.N / 2;
+    const int max_blocks = p.sorted_num / BM;
+    const int cap = tokn_cap(p);
+    int32_t *count = static_cast<int32_t *>(items);
+    int4 *items_end = static_cast<int4 *>(items) + 1 + 2 * static_cast<size_t>(max_blocks);
+    int2 *row_info = reinterpret_cast<int2 *>(items_end);
+    Args a{};
+    a.row_info = row_info;
+    a.out = static_cast<__nv_bfloat16 *>(p.out);
+    a.live_rows = p.live_rows;
+    a.items = items_end, a.item_count = count;
+    a.M = p.M, a.K = p.K, a.H = H;
+
+    CUtensorMap w1, w2, x64, x16, act64, act16, act_st;
+    constexpr auto BF16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    constexpr auto SW = CU_TENSOR_MAP_SWIZZLE_128B;
+    if (int rc = make_gate_up_map(&w1, p.w, p.E, H, p.K)) return rc;
+    if (int rc = make_tmap_2d(&w2, BF16, 2, p.w2, static_cast<uint64_t>(p.E) * p.K, H, 128, BK, SW, "w2")) return rc;
+    if (int rc = make_tmap_2d(&x64, BF16, 2, x_sorted, p.sorted_num, p.K, 64, BK, SW, "x_sorted")) return rc;
+    if (int rc = make_tmap_2d(&x16, BF16, 2, x_sorted, p.sorted_num, p.K, 16, BK, SW, "x_sorted (16 rows)")) return rc;
+    if (int rc = make_tmap_2d(&act64, BF16, 2, act, p.sorted_num, H, 64, BK, SW, "act")) return rc;
+    if (int rc = make_tmap_2d(&act16, BF16, 2, act, p.sorted_num, H, 16, BK, SW, "act (16 rows)")) return rc;
+    if (int rc = make_tmap_2d(&act_st, BF16, 2, act, p.sorted_num, H, CHUNK, BK, SW, "act (store)")) return rc;
+
+    const int sms = sm_count();
+    const bool pdl = pdl_enabled();
+    constexpr int kWarps = PLAN_THREADS / 32;
+    // 1 KB-aligned slots: weights + the rows one CTA loads (a piece's half, in boxes of 16 or 64 rows)
+    const uint32_t stage_bytes = A_BYTES + (cap / 2) * 128;
+    const long long max_items = std::min<long long>(2ll * max_blocks,
+                                                    (static_cast<long long>(p.M) * p.top_k + cap - 1) / cap + max_blocks);
+    if (phases & 1) {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.blockDim = dim3(PLAN_THREADS);
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl ? 1 : 0;
+        const auto *x = static_cast<const __nv_bfloat16 *>(p.x);
+        auto *xs = static_cast<__nv_bfloat16 *>(x_sorted);
+        // by token from 64 MB of activations on (half of L2), when the inverse (one int per pair) fits its region
+        if (static_cast<long long>(p.M) * p.K * 2 >= (64ll << 20) && p.top_k >= 2 && p.top_k <= 32 &&
+            static_cast<long long>(p.M) * p.top_k <= p.sorted_num) {
+            int32_t *inv = reinterpret_cast<int32_t *>(row_info + p.sorted_num);
+            cfg.gridDim = dim3(std::min(4 * sms, (p.sorted_num + PLAN_THREADS - 1) / PLAN_THREADS));
+            PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, row_info_kernel, p.sorted_ids, p.npp, p.topk_weights, p.M, p.top_k,
+                                            p.sorted_num, row_info, inv));
+            cfg.gridDim = dim3(1 + 3 * sms);
+            PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, gather_tokens_plan_kernel, x, xs, p.sorted_ids, p.expert_ids, p.npp,
+                                            static_cast<const int32_t *>(inv), p.M, p.K, p.top_k, p.sorted_num, cap, p.bpc,
+                                            items_end, count));
+        } else {
+            cfg.gridDim = dim3(1 + std::min(3 * sms, (p.sorted_num + kWarps - 1) / kWarps));
+            PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, gather_plan_kernel, x, xs, p.sorted_ids, p.expert_ids, p.npp,
+                                            p.topk_weights, p.M, p.K, p.top_k, p.sorted_num, cap, p.bpc, items_end, count,
+                                            row_info));
+        }
+    }
+    if (phases & 2) {
+        Args up = a;
+        up.use_pdl = (pdl && (phases & 1)) ? 1 : 0;
+        up.zero_out = 1;
+        if (int rc = launch<true>(w1, x64, x16, act_st, up, stage_bytes, max_items * (H / 128), stream)) return rc;
+    }
+    if (phases & 4) {
+        Args dn = a;
+        dn.use_pdl = (pdl && (phases & 2)) ? 1 : 0;
+        if (int rc = launch<false>(w2, act64, act16, act_st, dn, stage_bytes, max_items * ((p.K + 255) / 256), stream))
+            return rc;
+    }
+    return PMOE_OK;
+}
+
+int wait_ns_store_tokn(unsigned long long ns) {
+    PMOE_CUDA_OK(cudaMemcpyToSymbol(g_wait_ns, &ns, sizeof(ns)));
+    return PMOE_OK;
+}
+
+int status_fetch_tokn(int *value, bool reset) {
+    if (value) PMOE_CUDA_OK(cudaMemcpyFromSymbol(value, g_status_tokn, sizeof(int)));
+    if (reset) {
+        const int zero = 0;
+        PMOE_CUDA_OK(cudaMemcpyToSymbol(g_status_tokn, &zero, sizeof(int)));
+    }
+    return PMOE_OK;
+}
+
+}  // namespace pmoe

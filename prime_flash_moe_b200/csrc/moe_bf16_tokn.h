@@ -1,0 +1,26 @@
+// Interface of the token-N bf16 kernels (moe_bf16_tokn.cu) to the bf16 launcher (moe_bf16.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+
+namespace pmoe {
+
+struct ToknProblem {
+    const void *x, *w, *w2;
+    void *out;
+    const int32_t *sorted_ids, *expert_ids, *npp;
+    const float *topk_weights;
+    const int32_t *live_rows;   // optional, as in CallExtras
+    int top_k, M, K, N, E, sorted_num, bpc;
+};
+
+// bytes of the work-item list and the per-row tokens and weights for a routing table of `sorted_num` rows (16-byte aligned region)
+size_t tokn_items_bytes(int sorted_num);
+
+// act [sorted_num, N/2] bf16, x_sorted [sorted_num, K] bf16 and items are regions of the call's workspace; `phases` as
+// in phase_mask()
+int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, int phases, cudaStream_t stream);
+
+}  // namespace pmoe

@@ -1,0 +1,122 @@
+"""Token-N bf16 kernels (routed rows on the N side of the MMA): expert sizes at the edges of a work item.
+
+The reference is the same FFN in fp64; the kernels round the activation and the result to bf16 (2^-9 relative each).
+"""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def reference(x, w1, w2, ids, wts):
+    """Expert FFN of every token (one expert per token, ids >= E: none) in fp64."""
+    E, N = w1.shape[:2]
+    ref = torch.zeros(x.shape, dtype=torch.float64)
+    for e in range(E):
+        rows = (ids[:, 0] == e).nonzero().flatten()
+        gu = x[rows].double() @ w1[e].double().t()
+        act = torch.nn.functional.silu(gu[:, :N // 2]) * gu[:, N // 2:]
+        ref[rows] = wts[rows].double() * (act @ w2[e].double().t())
+    return ref
+
+
+def check(out, ref):
+    err = (out.double().cpu() - ref).norm() / ref.norm()
+    assert err < 2 ** -7, float(err)     # two bf16 roundings (activation, result)
+
+
+def run(counts, K, N, bpc, T_extra=0):
+    """counts[e] routed rows for expert e, one expert per token; T_extra tokens are routed nowhere (expert id E)."""
+    from prime_flash_moe_b200 import capi
+    E, T = len(counts), sum(counts) + T_extra
+    g = torch.Generator().manual_seed(K + N + T)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    w1 = (torch.randn(E, N, K, generator=g) / K ** 0.5).to(torch.bfloat16)
+    w2 = (torch.randn(E, K, N // 2, generator=g) / (N // 2) ** 0.5).to(torch.bfloat16)
+    ids = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)] +
+                    [torch.full((T_extra,), E, dtype=torch.int32)])
+    ids = ids[torch.randperm(T, generator=g)].view(T, 1).contiguous()
+    wts = torch.rand(T, 1, generator=g) + 0.5
+    s, e, n = capi.moe_align(ids.to(DEV), E, 128, bpc)
+    out = torch.full((T, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    capi.fused_moe_bf16(x.to(DEV), w1.to(DEV), w2.to(DEV), s, e, n, wts.to(DEV), out, 1, bpc=bpc)
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    check(out, reference(x, w1, w2, ids, wts))
+    assert torch.equal(out.cpu()[ids[:, 0] == E], torch.zeros(T_extra, K, dtype=torch.bfloat16))
+
+
+@pytest.fixture(autouse=True)
+def token_n(monkeypatch):
+    monkeypatch.setenv("PMOE_TOKN", "1")
+
+
+# few rows per expert: pieces of at most 64 rows; many: of at most 256
+@pytest.mark.parametrize("bpc", [1, 2])
+@pytest.mark.parametrize("counts", [(1, 0, 2, 0), (31, 32, 33), (63, 65, 0, 1), (127, 128, 129), (255, 256, 257),
+                                    (0, 513, 300), (640, 1, 0)])
+def test_expert_sizes_at_item_edges(counts, bpc):
+    run(counts, 256, 512, bpc, T_extra=3)
+
+
+# runs of more row blocks than the planner looks at in one go (512)
+@pytest.mark.parametrize("counts", [(67000,), (66000, 3), (100, 65700, 40), (65536, 65536 + 1)])
+def test_long_runs(counts):
+    run(counts, 128, 256, 1)
+
+
+@pytest.mark.parametrize("K,N", [(128, 256), (384, 256), (640, 768), (1152, 512)])   # one k-step pair, K % 256 == 128
+def test_matrix_sizes_at_tile_edges(K, N):
+    run((40, 0, 130, 7), K, N, 1)
+
+
+def test_an_expert_seen_in_separate_runs_and_holes_inside_a_block():
+    """A hand-made routing table: expert 0 in two separate runs, and a block whose rows are not contiguous."""
+    from prime_flash_moe_b200 import capi
+    K, N, E, T = 256, 512, 2, 300
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    w1 = (torch.randn(E, N, K, generator=g) / 16).to(torch.bfloat16)
+    w2 = (torch.randn(E, K, N // 2, generator=g) / 16).to(torch.bfloat16)
+    table = torch.full((4, 128), -1, dtype=torch.int32)
+    table[0] = torch.arange(128)
+    table[1, :20] = torch.arange(128, 148)
+    table[2, 5:128:2] = torch.arange(148, 210)         # holes
+    table[3, :90] = torch.arange(210, 300)
+    experts = torch.tensor([0, 1, 0, 0], dtype=torch.int32)
+    wts = torch.rand(T, 1, generator=g) + 0.5
+    out = torch.empty(T, K, dtype=torch.bfloat16, device=DEV)
+    capi.fused_moe_bf16(x.to(DEV), w1.to(DEV), w2.to(DEV), table.view(-1).to(DEV), experts.to(DEV),
+                        torch.tensor([512], dtype=torch.int32, device=DEV), wts.to(DEV), out, 1)
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    ids = torch.zeros(T, 1, dtype=torch.int32)
+    ids[128:148] = 1
+    check(out, reference(x, w1, w2, ids, wts))
+
+
+@pytest.mark.parametrize("top_k,K", [(2, 2176), (3, 4096)])
+def test_rows_gathered_token_by_token(top_k, K):
+    """From 64 MB of activations on x is copied to the sorted rows token by token; some pairs are routed nowhere, some
+    tokens not at all. The row-M kernels, which gather by row, give the expected result."""
+    import os
+    from prime_flash_moe_b200 import capi
+    N, E = 256, 40
+    T = (64 << 20) // (2 * K) + 5
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x = torch.randn(T, K, generator=g, device=DEV, dtype=torch.bfloat16)
+    w1 = torch.randn(E, N, K, generator=g, device=DEV, dtype=torch.bfloat16) * K ** -0.5
+    w2 = torch.randn(E, K, N // 2, generator=g, device=DEV, dtype=torch.bfloat16) * (N // 2) ** -0.5
+    ids = torch.rand(T, E + 3, generator=g, device=DEV).topk(top_k).indices.to(torch.int32)   # ids >= E: no expert
+    ids[7] = E
+    wts = torch.rand(T, top_k, generator=g, device=DEV)
+    s, e, n = capi.moe_align(ids.contiguous(), E, 128, 1)
+    outs = []
+    for mode in ("1", "0"):
+        os.environ["PMOE_TOKN"] = mode      # the fixture restores the variable
+        outs.append(capi.fused_moe_bf16(x, w1, w2, s, e, n, wts, torch.empty_like(x), top_k).float())
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    assert (outs[0] - outs[1]).norm() / outs[1].norm() < 2 ** -7     # bf16 sums of top_k results in another order
+    assert not outs[0][7].any()
