@@ -840,8 +840,11 @@ int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, const GArgs &g, cu
 }
 
 // PMOE_BWD_PAIRS: 0 = one-CTA kernel everywhere; 1 = weight-gradient GEMMs on CTA pairs; 2 = the row-space GEMMs as
-// well (measured: no gain, their odd-last-block launch eats it); unset (-1) = 1 when an expert has 256 routed rows or
-// more on average (below that the weight-gradient launches are bound by their stores and the pairs measured slower)
+// well; unset (-1) = chosen by the average routed rows per expert. Weight gradients: pairs from 512 rows on (backward and
+// forward together, us, without / with: 204 rows 1514 / 1604, 313 rows 2371 / 2685, 536 rows 613 / 608, 835 rows 1493 /
+// 1434, 1131 rows 602 / 492). Row space: only for wide layers from 1024 rows on, where the launch for the experts' odd
+// last blocks is small beside the pairs (N = 28672: recompute 1643 -> 1264 + 196, d_act 973 -> 777 + 124, d_xs 1709 ->
+// 1256 + 239; 764 rows 4491 / 4625).
 int pairs_mode() {
     const char *v = getenv("PMOE_BWD_PAIRS");
     return (v && v[0] >= '0' && v[0] <= '2') ? v[0] - '0' : -1;
@@ -994,8 +997,9 @@ extern "C" int pmoe_fused_moe_bf16_backward_ex(const void *x, const void *w1, co
 
     const int mask = g_bwd_mask;
     const int pm = pairs_mode();
-    const bool pairs = pm >= 0 ? pm >= 1 : static_cast<long long>(T) * top_k >= 256ll * E;   // weight gradients
-    const bool row_pairs = pm == 2;
+    const long long routed = static_cast<long long>(T) * top_k;
+    const bool pairs = pm >= 0 ? pm >= 1 : routed >= 512ll * E;                            // weight gradients
+    const bool row_pairs = pm >= 0 ? pm == 2 : N >= 8192 && routed >= 1024ll * E;
     const int copy_grid = 8 * sm_count();
     if (mask & 1) {
         PMOE_CUDA_OK(cudaMemsetAsync(inv, 0xFF, static_cast<size_t>(T) * top_k * sizeof(int32_t), stream));
