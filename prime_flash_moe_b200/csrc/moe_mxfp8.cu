@@ -182,6 +182,7 @@ __device__ __forceinline__ void issue_slot(uint32_t d, uint32_t a_smem, uint32_t
 __global__ void __launch_bounds__(256)
 gather_rows_mxfp8_kernel(const uint8_t *__restrict__ x, const uint8_t *__restrict__ x_scales,
                          uint8_t *__restrict__ x_sorted, uint8_t *__restrict__ xsf_tiles, const Args a) {
+    pdl_wait_primary();        // launched as a programmatic dependent of whatever the stream holds: the quantiser
     pdl_launch_dependents();   // the gate/up (or fused) kernel may set itself up; it waits for this grid before loading
     const int warps_per_cta = blockDim.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -196,12 +197,18 @@ gather_rows_mxfp8_kernel(const uint8_t *__restrict__ x, const uint8_t *__restric
         if (tok < 0 || tok >= a.M) continue;
         const int4 *src = reinterpret_cast<const int4 *>(x + static_cast<size_t>(tok) * a.K);
         int4 *dst = reinterpret_cast<int4 *>(x_sorted + static_cast<size_t>(row) * a.K);
+#pragma unroll 4
         for (int ch = lane; ch < chunks; ch += 32) dst[ch] = __ldg(src + ch);
         const int r = row & 127;
-        uint8_t *tiles = xsf_tiles + static_cast<size_t>(row >> 7) * (a.K / 128) * SF_TILE;
+        uint8_t *tiles = xsf_tiles + static_cast<size_t>(row >> 7) * (a.K / 128) * SF_TILE + (r & 31) * 16 + (r >> 5) * 4;
         const uint8_t *srow = x_scales + static_cast<size_t>(tok) * kblocks;
-        for (int kb = lane; kb < kblocks; kb += 32)
-            tiles[(kb >> 2) * SF_TILE + (r & 31) * 16 + (r >> 5) * 4 + (kb & 3)] = srow[kb];
+        // the four scales of a 128-wide K block are neighbours on both sides: one word each when x_scales is aligned
+        if ((reinterpret_cast<uintptr_t>(x_scales) & 3) == 0) {
+            const uint32_t *s4 = reinterpret_cast<const uint32_t *>(srow);
+            for (int kt = lane; kt < a.K / 128; kt += 32) *reinterpret_cast<uint32_t *>(tiles + kt * SF_TILE) = s4[kt];
+        } else {
+            for (int kb = lane; kb < kblocks; kb += 32) tiles[(kb >> 2) * SF_TILE + (kb & 3)] = srow[kb];
+        }
     }
 }
 
@@ -1267,9 +1274,17 @@ int run(const Problem &p, void *workspace, cudaStream_t stream) {
     const int a_mode = a_operand_mode();
     const bool lsu = p.split && p.bpc == 1 && a_mode == 2 && (reinterpret_cast<uintptr_t>(p.x_scales) & 3) == 0;
     if ((phases & 1) && !lsu) {
-        gather_rows_mxfp8_kernel<<<std::min(4 * sms, (p.sorted_num + 7) / 8), 256, 0, stream>>>(
-            static_cast<const uint8_t *>(p.x), static_cast<const uint8_t *>(p.x_scales), x_sorted, xsf, a);
-        PMOE_CUDA_OK(cudaGetLastError());
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(std::min(8 * sms, (p.sorted_num + 7) / 8));
+        cfg.blockDim = dim3(256);
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl_enabled() ? 1 : 0;
+        PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, gather_rows_mxfp8_kernel, static_cast<const uint8_t *>(p.x),
+                                        static_cast<const uint8_t *>(p.x_scales), x_sorted, xsf, a));
     }
     if (!p.split) {
         // memset(acc32) -> [gather] -> fused kernel -> out += bf16(acc32)

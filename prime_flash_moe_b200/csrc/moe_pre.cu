@@ -82,6 +82,7 @@ __device__ __forceinline__ uint32_t e4m3x4(float a, float b, float c, float d) {
 __global__ void __launch_bounds__(256)
 quantize_mx_kernel(const __nv_bfloat16 *__restrict__ x, const int32_t *__restrict__ row_index, int src_rows,
                    uint8_t *__restrict__ q, uint8_t *__restrict__ scales, int rows, int K) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the row gather may set itself up meanwhile
     const int kblocks = K / 32;
     const long long total = static_cast<long long>(rows) * kblocks;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
