@@ -327,7 +327,7 @@ __device__ __forceinline__ Tile fetch_tile(const int4 *items, int t, int num_til
     Tile w{0, 0, 0, 0};
     if (t < num_tiles) {
         const Coord c = tile_coord(t, n_items, n_tiles);
-        const int4 it = items[c.m_blk];
+        const int4 it = __ldcg(items + c.m_blk);
         w.expert = it.x, w.row0 = it.y, w.rows = it.z, w.n_tile = c.n_tile;
     }
     return w;
@@ -338,7 +338,7 @@ __device__ __forceinline__ void fetch_rows(const int2 *row_info, const Tile &w, 
     for (int j = 0; j < 4; ++j) {
         const int ch = grp + 2 * j;
         r[j] = make_int2(-1, 0);
-        if (ch * CHUNK < w.rows) r[j] = row_info[w.row0 + ch * CHUNK + lane];
+        if (ch * CHUNK < w.rows) r[j] = __ldcg(row_info + w.row0 + ch * CHUNK + lane);
     }
 }
 
@@ -387,11 +387,16 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(sm.tmem_slot()));
 
-    // a dependent CTA that shares this SM then blocks in its own TMEM allocation until this CTA has freed its columns
-    if (kUp) pdl_launch_dependents();
-    if (a.use_pdl) pdl_wait_primary();
+    // Gate/up: everything comes from the preparation. Its dependents are let go only now: a down CTA that starts knows
+    // that every gate/up CTA has passed this wait, hence that the items and row info are there, and that a CTA it shares
+    // an SM with holds its TMEM already (it blocks in its own allocation until those columns are freed). The down
+    // kernel's threads wait where they first touch what gate/up writes: activations and the zeroed `out`.
+    if (kUp) {
+        if (a.use_pdl) pdl_wait_primary();
+        pdl_launch_dependents();
+    }
 
-    const int n_items = *a.item_count;
+    const int n_items = __ldcg(a.item_count);
     const int4 *items = a.items - n_items;
     const int n_tiles = kUp ? a.H / 128 : (a.K + 255) / 256;
     const int num_tiles = n_items * n_tiles;
@@ -415,17 +420,26 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const int box = big ? 64 : 16;
                 const int boxes = (half + box - 1) / box;
                 const uint32_t bytes = 2 * (A_BYTES + static_cast<uint32_t>(boxes * box) * 128u);
+                auto load_weights = [&](int slot, int ks) {
+                    const uint32_t full_leader = mapa_shared(sm.full(slot), 0);
+                    if (leader) mbar_arrive_expect_tx(sm.full(slot), bytes);
+                    if (kUp)
+                        tma_load_5d_pair(sm.a(slot), &map_w, full_leader, ks * BK, 0, 0,
+                                         w.n_tile * 8 + static_cast<int>(rank) * 4, w.expert);
+                    else
+                        tma_load_2d_pair(sm.a(slot), &map_w, full_leader, ks * BK,
+                                         w.expert * a.K + w.n_tile * 256 + static_cast<int>(rank) * 128);
+                };
+                // down: the weights of the first round of slots do not depend on gate/up, only their rows do
+                const int early = !kUp && t == first ? min(a.stages, ksteps) : 0;
+                for (int ks = 0; ks < early; ++ks) load_weights(ks, ks);
+                const long long before = issued;
+                if (!kUp && t == first && a.use_pdl) pdl_wait_primary();
                 for (int ks = 0; ks < ksteps; ++ks) {
                     ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
                     if (!ok) break;
                     const uint32_t full_leader = mapa_shared(sm.full(s), 0);
-                    if (leader) mbar_arrive_expect_tx(sm.full(s), bytes);
-                    if (kUp)
-                        tma_load_5d_pair(sm.a(s), &map_w, full_leader, ks * BK, 0, 0,
-                                         w.n_tile * 8 + static_cast<int>(rank) * 4, w.expert);
-                    else
-                        tma_load_2d_pair(sm.a(s), &map_w, full_leader, ks * BK,
-                                         w.expert * a.K + w.n_tile * 256 + static_cast<int>(rank) * 128);
+                    if (ks >= early) load_weights(s, ks);
                     for (int j = 0; j < boxes; ++j)
                         tma_load_2d_pair(sm.b(s) + j * box * 128, big ? &map_rows64 : &map_rows16, full_leader, ks * BK,
                                          row0 + j * box);
@@ -435,6 +449,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         ph ^= 1;
                     }
                 }
+                if (!ok) issued = max(issued, before + early);
             }
             if (!ok && leader) {
                 // give the copies already issued (both CTAs' bytes arrive here) a bounded time to land
@@ -572,6 +587,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         Tile w, next = fetch(first);
         int2 info[4], info_next[4];
         if (!kUp) fetch_rows(a.row_info, next, grp, lane, info_next);
+        if (!kUp && a.use_pdl) pdl_wait_primary();
         for (int t = first; t < num_tiles && ok; t += step) {
             w = next;
             next = fetch(t + step);
