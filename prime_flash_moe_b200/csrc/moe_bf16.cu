@@ -1589,10 +1589,15 @@ Decisions decide(const Problem &p) {
     // A batch whose gate/up tiles fill the SMs once but not the CTA pairs (each pair would take a second, mostly empty
     // round) is left to the row-M kernels too when K is long (10 experts x 12 tiles, K = 3456: 67 / 70 us, but 18 x 8,
     // K = 2176: 59 / 57; 5 x 25, K = 1408: 59 / 51).
-    const long long tiles = std::min<long long>(p.E, static_cast<long long>(p.M) * p.top_k) * (p.N / 256);
+    // A narrow layer whose tiles fit one round of the CTA pairs is faster on the token-N kernels all the same: they split
+    // the long gate/up contraction's weights over two SMs (9 experts, K = 4992, N = 1024, 50 rows each: 70 / 57 us; 8
+    // experts, K = 4864, N = 512, 168 rows: 68 / 60; above one round 22 experts, N = 1024, 83 rows: 89 / 95).
+    const long long rows = static_cast<long long>(p.M) * p.top_k, experts = std::min<long long>(p.E, rows);
+    const long long tiles = experts * (p.N / 256);
     const bool second_round = 2 * tiles > sm_count() && tiles <= sm_count() && p.K >= 3072;
+    const bool one_round = 2 * (experts + rows / 256) * (p.N / 256) <= sm_count();
     d.token_n = token_n_enabled() && !call_extras().out_rows && !call_extras().gu_out &&
-                ((p.N > 1024 && !second_round) || token_n_forced());
+                ((p.N > 1024 && !second_round) || one_round || token_n_forced());
     return d;
 }
 
