@@ -1580,8 +1580,8 @@ Decisions decide(const Problem &p) {
         d.a_mode = (p.bpc == 1 && p.N < 8192 && static_cast<long long>(p.M) * p.top_k >= 256ll * p.E) ? 2 : 1;
     d.pregather = d.a_mode == 1 || p.bpc == 2;   // the CTA-pair kernels always take pre-gathered rows
     d.tails = p.bpc == 2 && pair_tails_enabled();
-    // results addressed through out_rows may live in a peer's memory (plain vector reductions only) and kept
-    // pre-activations are stored per accumulator row: both stay with the row-M kernels
+    // results addressed through out_rows may live in a peer's memory (plain vector reductions only): they stay with the
+    // row-M kernels
     // ... and so do the narrowest layers: the row-gathered copy of x and the short down tiles cost the token-N kernels
     // more than they gain there (row-M / token-N, us: N = 768, 949 rows per expert 187 / 228; N = 1024, 29 rows 152 / 168;
     // N = 1024, 2813 rows 3160 / 4080; but N = 1536, 512 rows 801 / 724; N = 2048, 1911 rows 319 / 282; N = 3072, Zipf
@@ -1596,7 +1596,7 @@ Decisions decide(const Problem &p) {
     const long long tiles = experts * (p.N / 256);
     const bool second_round = 2 * tiles > sm_count() && tiles <= sm_count() && p.K >= 3072;
     const bool one_round = 2 * (experts + rows / 256) * (p.N / 256) <= sm_count();
-    d.token_n = token_n_enabled() && !call_extras().out_rows && !call_extras().gu_out &&
+    d.token_n = token_n_enabled() && !call_extras().out_rows &&
                 ((p.N > 1024 && !second_round) || one_round || token_n_forced());
     return d;
 }
@@ -1703,6 +1703,7 @@ int run(const Problem &p, void *workspace, size_t workspace_bytes, cudaStream_t 
     const int phases = phase_mask();  // profiling hook: 1 = gather, 2 = gate/up, 4 = down (default all)
     if (dec.token_n) {
         const ToknProblem t{p.x, p.w, p.w2, p.out, p.sorted_ids, p.expert_ids, p.npp, p.topk_weights, extras.live_rows,
+                            extras.gu_out,
                             p.top_k, p.M, p.K, p.N, p.E, p.sorted_num, p.bpc};
         return run_tokn_bf16(t, workspace, ws_base + lay.x_sorted, ws_base + lay.items, phases, stream);
     }

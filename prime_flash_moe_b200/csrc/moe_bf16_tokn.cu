@@ -47,6 +47,9 @@ constexpr uint32_t UP_BUF_BYTES = CHUNK * 128;           // 32 rows x 64 activat
 constexpr uint32_t DOWN_ROW_BYTES = 256 + 16;            // 128 output columns, padded against bank conflicts
 constexpr uint32_t DOWN_BUF_BYTES = CHUNK * DOWN_ROW_BYTES;
 constexpr uint32_t UP_STAGING = 2 * UP_BUFS * UP_BUF_BYTES;       // 32 KB
+constexpr int KEEP_BUFS = 2;                                      // gate/up with kept pre-activations: activation, gate
+constexpr uint32_t KEEP_BUF_BYTES = 3 * UP_BUF_BYTES;             // and up chunks in one buffer
+constexpr uint32_t KEEP_STAGING = 2 * KEEP_BUFS * KEEP_BUF_BYTES; // 48 KB
 constexpr uint32_t DOWN_STAGING = 2 * DOWN_BUFS * DOWN_BUF_BYTES; // 51 KB
 constexpr uint32_t BAR_BYTES = 512;
 constexpr uint32_t SMEM_LIMIT = 232448;
@@ -76,10 +79,6 @@ struct Smem {
     __device__ __forceinline__ uint32_t freed(int i) const { return bars + 8 * (2 * MAX_STAGES + 4 + 2 * UP_BUFS + i); }
     __device__ __forceinline__ uint32_t tmem_slot() const { return bars + 8 * (2 * MAX_STAGES + 4 + 4 * UP_BUFS); }
 };
-
-size_t smem_bytes(int stages, uint32_t stage_bytes, bool up) {
-    return 1024 + static_cast<size_t>(stages) * stage_bytes + (up ? UP_STAGING : DOWN_STAGING) + BAR_BYTES;
-}
 
 __device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar_cluster_addr, int c0,
                                                  int c1, int c2, int c3, int c4) {
@@ -342,14 +341,15 @@ __device__ __forceinline__ void fetch_rows(const int2 *row_info, const Tile &w, 
     }
 }
 
-template <bool kUp>
+// kKeep: the gate/up kernel also stores the pre-activations (bf16, [sorted_num, N]) for a later backward pass
+template <bool kUp, bool kKeep = false>
 __global__ void __launch_bounds__(THREADS, 1)
 moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_rows64,
                 const __grid_constant__ CUtensorMap map_rows16, const __grid_constant__ CUtensorMap map_act,
-                const Args a) {
+                const __grid_constant__ CUtensorMap map_gu, const Args a) {
     extern __shared__ uint8_t smem_raw[];
-    constexpr int kBufs = kUp ? UP_BUFS : DOWN_BUFS;
-    constexpr uint32_t kBufBytes = kUp ? UP_BUF_BYTES : DOWN_BUF_BYTES;
+    constexpr int kBufs = !kUp ? DOWN_BUFS : kKeep ? KEEP_BUFS : UP_BUFS;
+    constexpr uint32_t kBufBytes = !kUp ? DOWN_BUF_BYTES : kKeep ? KEEP_BUF_BYTES : UP_BUF_BYTES;
     Smem sm;
     sm.stage_bytes = a.stage_bytes;
     sm.ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -551,6 +551,19 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 tmem_ld_wait();
                 if (!ok) break;
                 if (kUp) {
+                    if (kKeep) {
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) {
+                            stmatrix_x4_trans(base + UP_BUF_BYTES + p * 16 * 128, pack_bf16x2(lo[8 * p], lo[8 * p + 1]),
+                                              pack_bf16x2(lo[8 * p + 2], lo[8 * p + 3]),
+                                              pack_bf16x2(lo[8 * p + 4], lo[8 * p + 5]),
+                                              pack_bf16x2(lo[8 * p + 6], lo[8 * p + 7]));
+                            stmatrix_x4_trans(base + 2 * UP_BUF_BYTES + p * 16 * 128, pack_bf16x2(hi[8 * p], hi[8 * p + 1]),
+                                              pack_bf16x2(hi[8 * p + 2], hi[8 * p + 3]),
+                                              pack_bf16x2(hi[8 * p + 4], hi[8 * p + 5]),
+                                              pack_bf16x2(hi[8 * p + 6], hi[8 * p + 7]));
+                        }
+                    }
 #pragma unroll
                     for (int i = 0; i < 16; ++i) lo[i] = swiglu(lo[i], hi[i]);
 #pragma unroll
@@ -608,7 +621,13 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 ok = warp_wait(sm.staged(grp * kBufs + slot), round & 1, status, ST_TIMEOUT_ACT, lane);
                 if (!ok) break;
                 if (kUp) {
-                    if (lane == 0) tma_store_2d(&map_act, base, col0, w.row0 + ch * CHUNK);
+                    if (lane == 0) {
+                        tma_store_2d(&map_act, base, col0, w.row0 + ch * CHUNK);
+                        if (kKeep) {
+                            tma_store_2d(&map_gu, base + UP_BUF_BYTES, col0, w.row0 + ch * CHUNK);
+                            tma_store_2d(&map_gu, base + 2 * UP_BUF_BYTES, a.H + col0, w.row0 + ch * CHUNK);
+                        }
+                    }
                 } else if (info[j].x >= 0 && col0 < a.K) {
                     bulk_reduce_add_bf16(a.out + static_cast<size_t>(info[j].x) * a.K + col0, base + lane * DOWN_ROW_BYTES,
                                          256);
@@ -640,14 +659,14 @@ int make_gate_up_map(CUtensorMap *map, const void *w, int E, int H, int K) {
                         "w (gate | up interleaved)");
 }
 
-template <bool kUp>
-int launch(const CUtensorMap &mw, const CUtensorMap &m64, const CUtensorMap &m16, const CUtensorMap &mact, Args a,
-           uint32_t stage_bytes, long long max_tiles, cudaStream_t stream) {
+template <bool kUp, bool kKeep = false>
+int launch(const CUtensorMap &mw, const CUtensorMap &m64, const CUtensorMap &m16, const CUtensorMap &mact,
+           const CUtensorMap &mgu, Args a, uint32_t stage_bytes, long long max_tiles, cudaStream_t stream) {
     a.stage_bytes = stage_bytes;
-    const uint32_t fixed = 1024 + (kUp ? UP_STAGING : DOWN_STAGING) + BAR_BYTES;
+    const uint32_t fixed = 1024 + (!kUp ? DOWN_STAGING : kKeep ? KEEP_STAGING : UP_STAGING) + BAR_BYTES;
     a.stages = std::min<int>(MAX_STAGES, static_cast<int>((SMEM_LIMIT - fixed) / stage_bytes));
-    const size_t smem = smem_bytes(a.stages, stage_bytes, kUp);
-    auto kernel = moe_tokn_kernel<kUp>;
+    const size_t smem = fixed + static_cast<size_t>(a.stages) * stage_bytes;
+    auto kernel = moe_tokn_kernel<kUp, kKeep>;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -677,7 +696,7 @@ int launch(const CUtensorMap &mw, const CUtensorMap &m64, const CUtensorMap &m16
         pairs_of[dev].store(max_clusters, std::memory_order_release);
     }
     cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<long long>(max_tiles, max_clusters)));
-    PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, mw, m64, m16, mact, a));
+    PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, mw, m64, m16, mact, mgu, a));
     return PMOE_OK;
 }
 
@@ -763,12 +782,20 @@ int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, 
         Args up = a;
         up.use_pdl = (pdl && (phases & 1)) ? 1 : 0;
         up.zero_out = 1;
-        if (int rc = launch<true>(w1, x64, x16, act_st, up, stage_bytes, max_items * (H / 128), stream)) return rc;
+        const long long tiles = max_items * (H / 128);
+        if (p.gu_out) {
+            CUtensorMap gu_st;
+            if (int rc = make_tmap_2d(&gu_st, BF16, 2, p.gu_out, p.sorted_num, p.N, CHUNK, BK, SW, "gate | up (store)"))
+                return rc;
+            if (int rc = launch<true, true>(w1, x64, x16, act_st, gu_st, up, stage_bytes, tiles, stream)) return rc;
+        } else if (int rc = launch<true>(w1, x64, x16, act_st, act_st, up, stage_bytes, tiles, stream)) {
+            return rc;
+        }
     }
     if (phases & 4) {
         Args dn = a;
         dn.use_pdl = (pdl && (phases & 2)) ? 1 : 0;
-        if (int rc = launch<false>(w2, act64, act16, act_st, dn, stage_bytes, max_items * ((p.K + 255) / 256), stream))
+        if (int rc = launch<false>(w2, act64, act16, act_st, act_st, dn, stage_bytes, max_items * ((p.K + 255) / 256), stream))
             return rc;
     }
     return PMOE_OK;

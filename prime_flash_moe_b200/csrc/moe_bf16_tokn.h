@@ -13,6 +13,7 @@ struct ToknProblem {
     const int32_t *sorted_ids, *expert_ids, *npp;
     const float *topk_weights;
     const int32_t *live_rows;   // optional, as in CallExtras
+    void *gu_out;               // optional, as in CallExtras
     int top_k, M, K, N, E, sorted_num, bpc;
 };
 

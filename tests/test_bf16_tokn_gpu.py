@@ -120,3 +120,27 @@ def test_rows_gathered_token_by_token(top_k, K):
     assert capi.device_status() == 0
     assert (outs[0] - outs[1]).norm() / outs[1].norm() < 2 ** -7     # bf16 sums of top_k results in another order
     assert not outs[0][7].any()
+
+
+@pytest.mark.parametrize("counts", [(31, 0, 33), (257, 128, 5), (640, 70)])
+def test_kept_pre_activations(counts):
+    """gate | up of the routed rows in bf16, at the place of the row in the routing table."""
+    from prime_flash_moe_b200 import capi
+    K, N, E, T = 256, 768, len(counts), sum(counts)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    w1 = (torch.randn(E, N, K, generator=g) / 16).to(torch.bfloat16)
+    w2 = (torch.randn(E, K, N // 2, generator=g) / 20).to(torch.bfloat16)
+    ids = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)]).view(T, 1)
+    wts = torch.rand(T, 1, generator=g) + 0.5
+    s, e, n = capi.moe_align(ids.to(DEV), E, 128, 1)
+    out, gate_up = capi.fused_moe_bf16_keep(x.to(DEV), w1.to(DEV), w2.to(DEV), s, e, n, wts.to(DEV),
+                                            torch.empty(T, K, dtype=torch.bfloat16, device=DEV), 1)
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    check(out, reference(x, w1, w2, ids, wts))
+    rows = s.cpu().long()
+    kept = gate_up.cpu()[rows >= 0].double()
+    tok = rows[rows >= 0]
+    ref = torch.stack([w1[ids[t, 0]].double() @ x[t].double() for t in tok])
+    assert (kept - ref).norm() / ref.norm() < 2 ** -8      # one bf16 rounding
