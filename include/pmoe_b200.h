@@ -56,7 +56,8 @@ int pmoe_version(void);
  * num_experts <= 1024 as in the reference (fused_moe_bf16_kernel.cu:922-923).
  *
  * `pmoe_moe_align` takes its scratch from the stream-ordered allocator (cudaMallocAsync);
- * `pmoe_moe_align_ws` uses caller memory of at least `pmoe_moe_align_workspace_bytes` bytes
+ * `pmoe_moe_align_ws` uses caller memory of at least `pmoe_moe_align_workspace_bytes` bytes (up to 4096 ids, or 16384
+ * with at most 256 experts, may come without: one CTA then aligns them, more slowly)
  * (may be 0 for small n), 16-byte aligned, and performs no allocation. */
 int pmoe_moe_align(const int32_t *topk_ids, int32_t *sorted_token_ids, int32_t *expert_ids,
                    int32_t *num_tokens_post_padded, int n, int num_experts, int block_m, int pad_to,
@@ -186,10 +187,9 @@ enum { PMOE_DTYPE_F32 = 0, PMOE_DTYPE_BF16 = 1 };
 int pmoe_route_topk(const void *logits, int logits_dtype, int T, int num_experts, int top_k, int renormalize,
                     int32_t *topk_ids, float *topk_weights, pmoe_stream_t stream);
 /* Router and moe_align in one call: as pmoe_route_topk followed by pmoe_moe_align_ws on its topk_ids (same outputs,
- * bit for bit), but for n = T * top_k above the single-CTA sizes ONE kernel routes the tokens, counts its own ids
- * per expert and pre-fills sorted_token_ids - the ids are not read back for counting and one launch disappears.
- * workspace: pmoe_moe_align_workspace_bytes(T * top_k, num_experts) bytes. When top_k does not divide the id range
- * of a thread block (it does for every power of two up to 256) the two separate kernels run. */
+ * bit for bit); a decode batch (T <= 32) is routed and aligned by one launch.
+ * workspace: pmoe_moe_align_workspace_bytes(T * top_k, num_experts) bytes. Up to 4096 ids (16384 with at most 256
+ * experts) may come without: one CTA then aligns them, more slowly. */
 int pmoe_route_topk_align(const void *logits, int logits_dtype, int T, int num_experts, int top_k, int renormalize,
                           int32_t *topk_ids, float *topk_weights, int32_t *sorted_token_ids, int32_t *expert_ids,
                           int32_t *num_tokens_post_padded, int block_m, int pad_to, int max_padded, int max_blocks,

@@ -396,8 +396,9 @@ int launch(const int32_t *topk_ids, int32_t *sorted, int32_t *expert_ids, int32_
 namespace pmoe {
 namespace {
 
-// Decode batches: one CTA routes the tokens (one warp each, one or two rounds) and aligns the ids it still holds in
-// shared memory. T = 16, E = 128, top_k = 8: router 3.2 us + align 5.0 us + the gap between them 2.7 us before.
+// Decode batches: one CTA routes the tokens (one warp each) and aligns the ids it still holds in shared memory. One launch
+// instead of two: 8.0 us either way on the GPU at T = 16, E = 128, top_k = 8, but 5 us less of the host's 20 a call. With
+// more than one round of warps the single CTA loses (T = 64: 12.5 us against 8.0).
 constexpr int kOneCtaTokens = 32;      // one round of 32 warps (E <= 256); with 8 warps a quarter of it
 constexpr int kOneCtaExperts = 768;    // counters + ids fit 48 KB of shared memory
 
@@ -515,7 +516,7 @@ extern "C" int pmoe_moe_align(const int32_t *topk_ids, int32_t *sorted_token_ids
     if (int rc = check_args(topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, n, num_experts,
                             block_m, pad_to, max_padded, max_blocks))
         return rc;
-    const Plan p = make_plan(n, num_experts);
+    const Plan p = plan_with_scratch(n, num_experts, nullptr, 0);   // short problems allocate nothing
     int *ws = nullptr;
     if (p.ws_ints)
         if (int rc = scratch_alloc(reinterpret_cast<void **>(&ws), p.ws_ints * sizeof(int), stream)) return rc;
@@ -572,7 +573,7 @@ extern "C" int pmoe_moe_align_static(const int32_t *topk_ids, int32_t *sorted_to
     if (int rc = check_args(topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, n, num_experts,
                             block_m, pad_to, max_padded, max_blocks))
         return rc;
-    const Plan p = make_plan(n, num_experts);
+    const Plan p = plan_with_scratch(n, num_experts, nullptr, 0);   // short problems leave the shared array alone
     PMOE_REQUIRE(p.ws_ints <= kStaticScratchInts, PMOE_ERR_UNSUPPORTED,
                  "moe_align_static: n=%d with %d experts needs %zu bytes of scratch, the built-in array holds %zu; "
                  "use pmoe_moe_align_ws with caller memory instead",

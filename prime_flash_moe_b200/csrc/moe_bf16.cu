@@ -1584,20 +1584,24 @@ Decisions decide(const Problem &p) {
     // row-M kernels
     // ... and so do the narrowest layers: the row-gathered copy of x and the short down tiles cost the token-N kernels
     // more than they gain there (row-M / token-N, us: N = 768, 949 rows per expert 187 / 228; N = 1024, 29 rows 152 / 168;
-    // N = 1024, 2813 rows 3160 / 4080; but N = 1536, 512 rows 801 / 724; N = 2048, 1911 rows 319 / 282; N = 3072, Zipf
-    // over 4096 rows 18090 / 16670)
+    // N = 1024, 2813 rows 3160 / 4080; but N = 1536, 512 rows 801 / 724)
     // A batch whose gate/up tiles fill the SMs once but not the CTA pairs (each pair would take a second, mostly empty
     // round) is left to the row-M kernels too when K is long (10 experts x 12 tiles, K = 3456: 67 / 70 us, but 18 x 8,
     // K = 2176: 59 / 57; 5 x 25, K = 1408: 59 / 51).
     // A narrow layer whose tiles fit one round of the CTA pairs is faster on the token-N kernels all the same: they split
     // the long gate/up contraction's weights over two SMs (9 experts, K = 4992, N = 1024, 50 rows each: 70 / 57 us; 8
     // experts, K = 4864, N = 512, 168 rows: 68 / 60; above one round 22 experts, N = 1024, 83 rows: 89 / 95).
+    // From 1024 rows per expert on padding to 128 rows costs little, and the two-block kernel that gathers the rows itself
+    // saves the row-gathered copy in HBM, whose power counts on a chip at its cap: it stays where the rows are long beside
+    // the layer's width (row-M / token-N: K = 4096, N = 3072, 524288 Zipf rows 18.8 / 20.0 ms at the cap, though 18.1 /
+    // 16.7 ms on a cool chip; K = 2688, N = 1280 1916 / 2010 us; but K = 2304, N = 2816 4294 / 3878 us; K = 5248, N = 5120
+    // 2428 / 1961; K = 2176, N = 2048 319 / 282).
     const long long rows = static_cast<long long>(p.M) * p.top_k, experts = std::min<long long>(p.E, rows);
     const long long tiles = experts * (p.N / 256);
     const bool second_round = 2 * tiles > sm_count() && tiles <= sm_count() && p.K >= 3072;
     const bool one_round = 2 * (experts + rows / 256) * (p.N / 256) <= sm_count();
     d.token_n = token_n_enabled() && !call_extras().out_rows &&
-                ((p.N > 1024 && !second_round) || one_round || token_n_forced());
+                ((p.N > 1024 && !second_round && (8ll * p.K <= 9ll * p.N || rows < 1024ll * p.E)) || one_round || token_n_forced());
     return d;
 }
 

@@ -246,12 +246,13 @@ moe_up_mxfp8_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(sm.tmem_slot()));
 
+    if (a.use_pdl) pdl_wait_primary();   // launched as a programmatic dependent of the row-gather kernel
+
     // Dependents may be scheduled only now that this CTA holds its tensor memory: a dependent CTA that
     // shares this SM then blocks in its own allocation until this CTA has freed its columns, never the
-    // other way round (it still waits for this whole grid before it reads any result).
+    // other way round. It still waits for this whole grid before it reads any result, but not for the routing
+    // table: every CTA here has passed the wait above.
     pdl_launch_dependents();
-
-    if (a.use_pdl) pdl_wait_primary();   // launched as a programmatic dependent of the row-gather kernel
 
     const int m_blocks = live_row_blocks(a.npp, a.sorted_num);
     const int n_tiles = a.H / 128;
@@ -486,8 +487,6 @@ moe_down_mxfp8_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(sm.tmem_slot()));
 
-    if (a.use_pdl) pdl_wait_primary();
-
     const int m_blocks = live_row_blocks(a.npp, a.sorted_num);
     const int n_tiles = a.K / 256;
     const int num_tiles = m_blocks * n_tiles;
@@ -507,21 +506,31 @@ moe_down_mxfp8_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_
                 const uint8_t *sf_w1 = sf_w0 + static_cast<size_t>(ksteps) * SF_TILE;
                 const uint8_t *sf_a = a.act_sf + static_cast<size_t>(c.m_blk) * ksteps * SF_TILE;
                 const bool short_a = block_is_short(a, c.m_blk);
+                auto load_weights = [&](int slot, int ks) {
+                    mbar_arrive_expect_tx(sm.full(slot), short_a ? STAGE_TX_BYTES - A_BYTES + SHORT_A_BYTES : STAGE_TX_BYTES);
+                    tma_load_2d(sm.b(slot), &map_w2, sm.full(slot), ks * BKB, w2_row);
+                    bulk_load_1d(sm.sfb(slot), sf_w0 + static_cast<size_t>(ks) * SF_TILE, SF_TILE, sm.full(slot));
+                    bulk_load_1d(sm.sfb(slot) + SF_TILE, sf_w1 + static_cast<size_t>(ks) * SF_TILE, SF_TILE, sm.full(slot));
+                };
+                // the weights of the first round of slots do not depend on gate/up: issued before the wait for it
+                const bool first_tile = t == static_cast<int>(blockIdx.x);
+                const int early = first_tile ? min(a.stages, ksteps) : 0;
+                for (int ks = 0; ks < early; ++ks) load_weights(ks, ks);
+                if (first_tile && a.use_pdl) pdl_wait_primary();
+                const long long before = issued;
                 for (int ks = 0; ks < ksteps; ++ks) {
                     ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
                     if (!ok) break;
-                    mbar_arrive_expect_tx(sm.full(s), short_a ? STAGE_TX_BYTES - A_BYTES + SHORT_A_BYTES : STAGE_TX_BYTES);
+                    if (ks >= early) load_weights(s, ks);
                     tma_load_2d(sm.a(s), short_a ? &map_act_short : &map_act, sm.full(s), ks * BKB, c.m_blk * BM);
-                    tma_load_2d(sm.b(s), &map_w2, sm.full(s), ks * BKB, w2_row);
                     bulk_load_1d(sm.sfa(s), sf_a + static_cast<size_t>(ks) * SF_TILE, SF_TILE, sm.full(s));
-                    bulk_load_1d(sm.sfb(s), sf_w0 + static_cast<size_t>(ks) * SF_TILE, SF_TILE, sm.full(s));
-                    bulk_load_1d(sm.sfb(s) + SF_TILE, sf_w1 + static_cast<size_t>(ks) * SF_TILE, SF_TILE, sm.full(s));
                     ++issued;
                     if (++s == a.stages) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
+                if (!ok) issued = max(issued, before + early);
             }
             if (!ok) drain_fills(sm, a.stages, issued);
         }
@@ -559,6 +568,7 @@ moe_down_mxfp8_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_
         const uint32_t lane_base = (warp & 3) * 32;
         const int row = lane_base + lane;
         const int cg = ew >> 2;          // output columns [cg*128, cg*128+128) of the 256-wide tile
+        if (a.use_pdl) pdl_wait_primary();   // gate/up zeroes `out`
         int it = 0;
         for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
             const Coord c = tile_coord(t, m_blocks, n_tiles);

@@ -31,7 +31,7 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 // that ties keep the lower index first); a round is a warp maximum over the heads, and its owner (of several, the one
 // with the lowest index) moves its list up by one. Returns false, with nothing selected, when fewer than
 // top_k logits are above -inf: the general loop below then decides.
-// Against the general loop (8192 tokens, E = 128, top_k = 8): router 23 -> 8 us.
+// 65536 tokens, E = 128, top_k = 8, router and align: 112.7 us with the general loop, 101.9 with this one.
 template <typename T, int PER>
 __device__ __forceinline__ bool select_sorted(const float (&v)[PER], int E, int top_k, int lane, float &my_val, int &my_idx,
                                               float &row_max) {
@@ -60,7 +60,7 @@ __device__ __forceinline__ bool select_sorted(const float (&v)[PER], int E, int 
         const uint32_t kmax = __reduce_max_sync(kFull, key[0]);
         if (kmax <= kMinusInf) return false;
         if (j == 0) row_max = key_float(kmax);
-        // one owner in all but tied rounds; redux is the slow instruction here, a vote and a shuffle are not
+        // one owner in all but tied rounds
         const unsigned owners = __ballot_sync(kFull, key[0] == kmax);
         int e_win = __shfl_sync(kFull, idx[0], __ffs(owners) - 1);
         if (owners & (owners - 1)) e_win = __reduce_min_sync(kFull, key[0] == kmax ? idx[0] : 0x7fffffff);

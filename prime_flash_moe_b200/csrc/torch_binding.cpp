@@ -262,14 +262,15 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, torch::Te
     torch::Tensor sorted = torch::empty({max_padded}, i32), experts = torch::empty({max_padded / block_m}, i32);
     torch::Tensor npp = torch::empty({1}, i32);
     const size_t ws_bytes = pmoe_moe_align_workspace_bytes(static_cast<int>(n), static_cast<int>(E));
-    torch::Tensor ws = torch::empty({static_cast<int64_t>(ws_bytes) + 16}, logits.options().dtype(torch::kUInt8));
+    torch::Tensor ws;
+    if (ws_bytes) ws = torch::empty({static_cast<int64_t>(ws_bytes)}, logits.options().dtype(torch::kUInt8));
     check_status(pmoe_route_topk_align(
         logits.const_data_ptr(), logits.dtype() == torch::kFloat32 ? PMOE_DTYPE_F32 : PMOE_DTYPE_BF16, static_cast<int>(T),
         static_cast<int>(E), static_cast<int>(top_k), renormalize ? 1 : 0, static_cast<int32_t *>(ids.data_ptr()),
         static_cast<float *>(wts.data_ptr()), static_cast<int32_t *>(sorted.data_ptr()),
         static_cast<int32_t *>(experts.data_ptr()), static_cast<int32_t *>(npp.data_ptr()), static_cast<int>(block_m),
-        static_cast<int>(pad_to), static_cast<int>(max_padded), static_cast<int>(max_padded / block_m), ws.data_ptr(),
-        ws_bytes, stream));
+        static_cast<int>(pad_to), static_cast<int>(max_padded), static_cast<int>(max_padded / block_m),
+        ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream));
     return {ids, wts, sorted, experts, npp};
 }
 
