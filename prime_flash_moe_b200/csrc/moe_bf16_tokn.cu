@@ -233,6 +233,15 @@ gather_plan_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restric
     }
     const int lane = threadIdx.x & 31;
     const int rows = blocks * BM;
+    if (!x_sorted) {     // a phase mask without the row copy: only the row info
+        for (int row = (blockIdx.x - 1) * PLAN_THREADS + threadIdx.x; row < rows; row += (gridDim.x - 1) * PLAN_THREADS) {
+            const int pair = sorted_ids[row];
+            const int tok = pair >= 0 ? pair / top_k : -1;
+            const bool live = tok >= 0 && tok < M;
+            row_info[row] = make_int2(live ? tok : -1, live ? __float_as_int(topk_weights[pair]) : 0);
+        }
+        return;
+    }
     const int chunks = K / 8;
     constexpr int kWarps = PLAN_THREADS / 32;
     for (int row = (blockIdx.x - 1) * kWarps + (threadIdx.x >> 5); row < rows; row += (gridDim.x - 1) * kWarps) {
@@ -736,8 +745,10 @@ int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, 
     constexpr auto SW = CU_TENSOR_MAP_SWIZZLE_128B;
     if (int rc = make_gate_up_map(&w1, p.w, p.E, H, p.K)) return rc;
     if (int rc = make_tmap_2d(&w2, BF16, 2, p.w2, static_cast<uint64_t>(p.E) * p.K, H, 128, BK, SW, "w2")) return rc;
-    if (int rc = make_tmap_2d(&x64, BF16, 2, x_sorted, p.sorted_num, p.K, 64, BK, SW, "x_sorted")) return rc;
-    if (int rc = make_tmap_2d(&x16, BF16, 2, x_sorted, p.sorted_num, p.K, 16, BK, SW, "x_sorted (16 rows)")) return rc;
+    if (x_sorted) {
+        if (int rc = make_tmap_2d(&x64, BF16, 2, x_sorted, p.sorted_num, p.K, 64, BK, SW, "x_sorted")) return rc;
+        if (int rc = make_tmap_2d(&x16, BF16, 2, x_sorted, p.sorted_num, p.K, 16, BK, SW, "x_sorted (16 rows)")) return rc;
+    }
     if (int rc = make_tmap_2d(&act64, BF16, 2, act, p.sorted_num, H, 64, BK, SW, "act")) return rc;
     if (int rc = make_tmap_2d(&act16, BF16, 2, act, p.sorted_num, H, 16, BK, SW, "act (16 rows)")) return rc;
     if (int rc = make_tmap_2d(&act_st, BF16, 2, act, p.sorted_num, H, CHUNK, BK, SW, "act (store)")) return rc;
@@ -749,7 +760,9 @@ int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, 
     const uint32_t stage_bytes = A_BYTES + (cap / 2) * 128;
     const long long max_items = std::min<long long>(2ll * max_blocks,
                                                     (static_cast<long long>(p.M) * p.top_k + cap - 1) / cap + max_blocks);
-    if (phases & 1) {
+    // The work items and the row info are built in every call, also in one whose phase mask leaves the row copy out:
+    // the kernels below index with them.
+    {
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -759,9 +772,9 @@ int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, 
         cfg.attrs = attr;
         cfg.numAttrs = pdl ? 1 : 0;
         const auto *x = static_cast<const __nv_bfloat16 *>(p.x);
-        auto *xs = static_cast<__nv_bfloat16 *>(x_sorted);
+        auto *xs = (phases & 1) ? static_cast<__nv_bfloat16 *>(x_sorted) : nullptr;
         // by token from 64 MB of activations on (half of L2), when the inverse (one int per pair) fits its region
-        if (static_cast<long long>(p.M) * p.K * 2 >= (64ll << 20) && p.top_k >= 2 && p.top_k <= 32 &&
+        if (xs && static_cast<long long>(p.M) * p.K * 2 >= (64ll << 20) && p.top_k >= 2 && p.top_k <= 32 &&
             static_cast<long long>(p.M) * p.top_k <= p.sorted_num) {
             int32_t *inv = reinterpret_cast<int32_t *>(row_info + p.sorted_num);
             cfg.gridDim = dim3(std::min(4 * sms, (p.sorted_num + PLAN_THREADS - 1) / PLAN_THREADS));
@@ -780,7 +793,7 @@ int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, 
     }
     if (phases & 2) {
         Args up = a;
-        up.use_pdl = (pdl && (phases & 1)) ? 1 : 0;
+        up.use_pdl = pdl ? 1 : 0;
         up.zero_out = 1;
         const long long tiles = max_items * (H / 128);
         if (p.gu_out) {
