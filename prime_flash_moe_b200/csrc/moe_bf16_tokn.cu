@@ -233,7 +233,7 @@ gather_plan_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restric
     }
     const int lane = threadIdx.x & 31;
     const int rows = blocks * BM;
-    if (!x_sorted) {     // a phase mask without the row copy: only the row info
+    if (!x_sorted) {     // no row copy (another gate/up kernel, or a phase mask without it): only the row info
         for (int row = (blockIdx.x - 1) * PLAN_THREADS + threadIdx.x; row < rows; row += (gridDim.x - 1) * PLAN_THREADS) {
             const int pair = sorted_ids[row];
             const int tok = pair >= 0 ? pair / top_k : -1;

@@ -21,7 +21,7 @@ struct ToknProblem {
 size_t tokn_items_bytes(int sorted_num);
 
 // act [sorted_num, N/2] bf16, x_sorted [sorted_num, K] bf16 and items are regions of the call's workspace; `phases` as
-// in phase_mask().
+// in phase_mask(). x_sorted == nullptr (phase 4 only): another gate/up kernel has run, which gathers its rows itself
 int run_tokn_bf16(const ToknProblem &p, void *act, void *x_sorted, void *items, int phases, cudaStream_t stream);
 
 }  // namespace pmoe
