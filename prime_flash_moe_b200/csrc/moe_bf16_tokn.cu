@@ -149,10 +149,10 @@ __device__ void plan_items(const int32_t *__restrict__ sorted_ids, const int32_t
     __shared__ int s_sum[kWarps];
     __shared__ int s_ext[PLAN_THREADS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int next_chunk = blocks;   // first run start after this chunk ...
-    int next_ext = 0;          // ... and the extent of the block before it
+    int next_chunk = blocks;   // first run start after this chunk (or the end of the table) ...
+    int next_ext = 0;          // ... and the extent of the block before it, taken in the chunk that holds that block
     int written = 0;           // items of the later chunks
-    for (int c0 = (blocks - 1) / PLAN_THREADS * PLAN_THREADS; c0 >= 0; c0 -= PLAN_THREADS) {
+    for (int c0 = (blocks + PLAN_THREADS - 1) / PLAN_THREADS * PLAN_THREADS - PLAN_THREADS; c0 >= 0; c0 -= PLAN_THREADS) {
         const int b = c0 + threadIdx.x;
         block_extents(sorted_ids, c0, blocks, s_ext);
         bool start = false;
@@ -165,6 +165,8 @@ __device__ void plan_items(const int32_t *__restrict__ sorted_ids, const int32_t
         const uint32_t m = __ballot_sync(0xffffffffu, start);
         if (lane == 0) s_first[warp] = m ? c0 + warp * 32 + __ffs(m) - 1 : 0x7fffffff;
         __syncthreads();
+        // that block is in this chunk: at the table's end, or where a run starts at the very next chunk's first block
+        if (next_chunk <= c0 + PLAN_THREADS) next_ext = s_ext[next_chunk - 1 - c0];
         int next = next_chunk, first = next_chunk;
         for (int w = kWarps - 1; w >= 0; --w) {
             const int f = s_first[w];
@@ -204,12 +206,8 @@ __device__ void plan_items(const int32_t *__restrict__ sorted_ids, const int32_t
             }
         }
         written += total;
-        // a run of an earlier chunk that reaches into this one ends before this one's first run start, or at the end
-        if (first < next_chunk) {
-            if (first > c0) next_ext = s_ext[first - 1 - c0];
-        } else if (blocks > c0 && blocks <= c0 + PLAN_THREADS) {
-            next_ext = s_ext[blocks - 1 - c0];
-        }
+        // a run of an earlier chunk that reaches into this one ends before this one's first run start
+        if (first < next_chunk && first > c0) next_ext = s_ext[first - 1 - c0];
         next_chunk = first;
         __syncthreads();
     }

@@ -22,8 +22,9 @@ def reference(x, w1, w2, ids, wts):
 
 
 def check(out, ref):
-    err = (out.double().cpu() - ref).norm() / ref.norm()
-    assert err < 2 ** -7, float(err)     # two bf16 roundings (activation, result)
+    """Row by row: one norm over all rows does not see a few lost ones."""
+    err = (out.double().cpu() - ref).norm(dim=1) / ref.norm(dim=1).clamp_min(1e-30)
+    assert err.max() < 2 ** -7, (float(err.max()), int(err.argmax()))     # two bf16 roundings (activation, result)
 
 
 def run(counts, K, N, bpc, T_extra=0):
@@ -60,8 +61,10 @@ def test_expert_sizes_at_item_edges(counts, bpc):
     run(counts, 256, 512, bpc, T_extra=3)
 
 
-# runs of more row blocks than the planner looks at in one go (512)
-@pytest.mark.parametrize("counts", [(67000,), (66000, 3), (100, 65700, 40), (65536, 65536 + 1)])
+# runs of more row blocks than the planner looks at in one go (512); in the last two a run starts before such a chunk,
+# covers all of it and ends where the next one begins, with a partly filled block
+@pytest.mark.parametrize("counts", [(67000,), (66000, 3), (100, 65700, 40), (65536, 65536 + 1), (131044, 2000, 2000),
+                                    (100, 130893, 300)])
 def test_long_runs(counts):
     run(counts, 128, 256, 1)
 
