@@ -275,8 +275,9 @@ row_info_kernel(const int32_t *__restrict__ sorted_ids, const int32_t *__restric
     }
 }
 
-// CTA 0 builds the work items; in the others one warp per token. inv is not initialised: an entry counts only if the row it names holds that very pair (pairs that
-// the routing table leaves out have no row).
+// CTA 0 builds the work items; in the others one warp per token. inv is not initialised: an entry counts only if the row
+// it names holds that very pair (pairs that the routing table leaves out have no row). A caller's table may list a pair in
+// several rows, of which inv names one: the others are found in a pass over the rows and copied one by one.
 __global__ void __launch_bounds__(PLAN_THREADS)
 gather_tokens_plan_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ x_sorted,
                           const int32_t *__restrict__ sorted_ids, const int32_t *__restrict__ expert_ids,
@@ -318,6 +319,17 @@ gather_tokens_plan_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__
                     if (c < chunks) dst[c] = v[i];
                 }
             }
+        }
+    }
+    for (int r0 = ((blockIdx.x - 1) * kWarps + (threadIdx.x >> 5)) * 32; r0 < rows; r0 += (gridDim.x - 1) * kWarps * 32) {
+        const int pair = sorted_ids[r0 + lane];      // rows is a multiple of 128
+        const int tok = pair >= 0 ? pair / top_k : -1;
+        const bool other = tok >= 0 && tok < M && inv[pair] != r0 + lane;
+        for (uint32_t m = __ballot_sync(0xffffffffu, other); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const int4 *src = reinterpret_cast<const int4 *>(x + static_cast<size_t>(__shfl_sync(0xffffffffu, tok, l)) * K);
+            int4 *dst = reinterpret_cast<int4 *>(x_sorted + static_cast<size_t>(r0 + l) * K);
+            for (int c = lane; c < chunks; c += 32) dst[c] = __ldg(src + c);
         }
     }
 }
