@@ -28,7 +28,7 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 }
 
 // top-k of one token for PER <= 8 logits per lane, none of them NaN: every lane sorts its own logits once (stable, so
-// that ties keep the lower index first); a round is a warp maximum over the heads, and its owner (of several, the one
+// that ties, -0 and +0 among them, keep the lower index first as in the general loop); a round is a warp maximum over the heads, and its owner (of several, the one
 // with the lowest index) moves its list up by one. Returns false, with nothing selected, when fewer than
 // top_k logits are above -inf: the general loop below then decides.
 // 65536 tokens, E = 128, top_k = 8, router and align: 112.7 us with the general loop, 101.9 with this one.
@@ -37,6 +37,7 @@ __device__ __forceinline__ bool select_sorted(const float (&v)[PER], int E, int 
                                               float &row_max) {
     constexpr unsigned kFull = 0xffffffffu;
     constexpr uint32_t kMinusInf = 0x007fffffu;    // float_key(-inf); emptied slots and e >= E hold 0
+    constexpr uint32_t kMinusZero = 0x7fffffffu;   // float_key(-0.f), one below float_key(+0.f)
     uint32_t key[PER];
     int idx[PER];
     bool nan = false;
@@ -51,7 +52,7 @@ __device__ __forceinline__ bool select_sorted(const float (&v)[PER], int E, int 
     for (int n = PER - 1; n > 0; --n)
 #pragma unroll
         for (int i = 0; i < n; ++i) {
-            const bool swap = key[i] < key[i + 1];
+            const bool swap = key[i] + (key[i] == kMinusZero) < key[i + 1];
             const uint32_t k0 = swap ? key[i + 1] : key[i], k1 = swap ? key[i] : key[i + 1];
             const int i0 = swap ? idx[i + 1] : idx[i], i1 = swap ? idx[i] : idx[i + 1];
             key[i] = k0, key[i + 1] = k1, idx[i] = i0, idx[i + 1] = i1;

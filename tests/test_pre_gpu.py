@@ -218,3 +218,19 @@ def test_route_topk_ties_and_masked_logits(E, k):
         assert ids[t].tolist() == order, t
     ref = torch.softmax(torch.gather(logits, 1, ids.cpu().long()), -1)
     torch.testing.assert_close(wts.cpu(), ref, rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("T", [5, 200])        # routed and aligned in one launch / by the router's own
+@pytest.mark.parametrize("E", [40, 100, 250, 300])        # 2, 4, 8 and 16 logits per lane
+def test_route_topk_signed_zeros(T, E):
+    """-0 and +0 held by one lane (experts 32 apart) are a tie like any other: the lower expert comes first."""
+    import prime_flash_moe_b200 as P
+    logits = torch.full((T, E), -1.0)
+    logits[:, 3], logits[:, 35] = -0.0, 0.0
+    logits[::2, 3], logits[::2, 35] = 0.0, -0.0
+    logits[1, 3], logits[1, 35] = -0.0, 1e-38
+    ids, wts = P.route_topk_align(logits.to(DEV), 2)[:2]
+    want = torch.tensor([[3, 35]], dtype=torch.int32).repeat(T, 1)
+    want[1] = torch.tensor([35, 3])
+    assert torch.equal(ids.cpu(), want)
+    torch.testing.assert_close(wts.cpu(), torch.full((T, 2), 0.5), rtol=1e-6, atol=0)
