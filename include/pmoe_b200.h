@@ -356,6 +356,11 @@ int pmoe_debug_wait_probe(pmoe_stream_t stream);
 size_t pmoe_debug_bf16_workspace_extent(int M, int K, int N, int num_experts, int top_k, int sorted_num, int bpc,
                                         int split);
 
+/* Test hook: the kernels the bf16 split launcher would take for this problem under the current environment, as a sum of
+ * the values below (0: one row block per tile, row-M kernels). Host only, no device work. */
+enum { PMOE_ROUTE_TOKEN_N_UP = 1, PMOE_ROUTE_TOKEN_N_DOWN = 2, PMOE_ROUTE_TWO_BLOCK_UP = 4, PMOE_ROUTE_CTA_PAIRS = 8 };
+int pmoe_debug_bf16_route(int M, int K, int N, int num_experts, int top_k, int bpc, int with_live_rows);
+
 #ifdef __cplusplus
 }
 #endif

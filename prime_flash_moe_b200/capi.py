@@ -61,6 +61,7 @@ SIGNATURES = {
     "pmoe_debug_set_wait_ns": (_i, [C.c_ulonglong]),
     "pmoe_debug_wait_probe": (_i, [_vp]),
     "pmoe_debug_bf16_workspace_extent": (_sz, [_i] * 8),
+    "pmoe_debug_bf16_route": (_i, [_i] * 7),
 }
 
 _lib = None

@@ -1567,6 +1567,8 @@ struct Decisions {
     bool pregather;   // x_sorted region written and read
     bool tails;       // bpc == 2: pair / tail lists written and read
     bool token_n;     // the token-N kernels run instead (x_sorted and the work items written and read)
+    bool dual;        // bpc == 1, not token_n: two row blocks per gate/up tile (shared weight slots)
+    bool token_n_down;   // ... and the token-N down kernel after it (work items written and read)
 };
 Decisions decide(const Problem &p) {
     Decisions d{};
@@ -1602,6 +1604,17 @@ Decisions decide(const Problem &p) {
     const bool one_round = 2 * (experts + rows / 256) * (p.N / 256) <= sm_count();
     d.token_n = token_n_enabled() && !call_extras().out_rows &&
                 ((p.N > 1024 && !second_round && (8ll * p.K <= 9ll * p.N || rows < 1024ll * p.E)) || one_round || token_n_forced());
+    // PMOE_DUAL=0/1, unset = two blocks for calls with >= 1024 routed rows per expert on average (measured: gate/up
+    // kernel -4..-5 % there with the in-kernel gather, -13..-15 % when fed by TMA from the row-gathered copy; +5 % at 512
+    // rows per expert, where more pairs straddle two experts)
+    const int dual_env = dual_blocks_mode();
+    d.dual = p.bpc == 1 && !d.token_n && d.a_mode != 0 && (dual_env < 0 ? rows >= 1024ll * p.E : dual_env != 0);
+    // The two-block gate/up kernel hands its activations to the token-N down kernel where that saves more than the launch
+    // for its work items costs, about 15 us: on layers of N >= 2048 (whole call, us, without / with: K = 4096, N = 3072,
+    // 524288 rows 18600 / 17700; N = 2560, 16 experts, 1100 rows each, K = 5120 741 / 701; N = 2048, K = 5120 546 / 535;
+    // but N = 1536, K = 2048 177 / 193; N = 1280, K = 2560 195 / 218). Not with live_rows: M is then the capacity of a
+    // buffer of which few rows may be in use (capacity 8192, 32 rows in use, K = 4096, N = 3072: 247 / 265).
+    d.token_n_down = d.dual && p.N >= 2048 && token_n_enabled() && !call_extras().out_rows && !call_extras().live_rows;
     return d;
 }
 
@@ -1846,17 +1859,9 @@ int run(const Problem &p, void *workspace, size_t workspace_bytes, cudaStream_t 
         }
         return PMOE_OK;
     }
-    // two row blocks per tile (shared weight slots): PMOE_DUAL=0/1, unset = for calls with >= 1024 routed rows per
-    // expert on average (measured: gate/up kernel -4..-5 % there with the in-kernel gather, -13..-15 % when fed by
-    // TMA from the row-gathered copy; +5 % at 512 rows per expert, where more pairs straddle two experts)
-    const int dual_env = dual_blocks_mode();
-    const bool dual = a_mode != 0 && (dual_env < 0 ? static_cast<long long>(p.M) * p.top_k >= 1024ll * p.E : dual_env != 0);
-    // The two-block gate/up kernel hands its activations to the token-N down kernel (524288 rows, K = 4096, N = 3072: down
-    // 6.7 ms against 5.2, the call 18.6 against 17.7).
-    const bool token_n_down = dual && p.N > 1024 && token_n_enabled() && !extras.out_rows;
     const ToknProblem tdown{p.x, p.w, p.w2, p.out, p.sorted_ids, p.expert_ids, p.npp, p.topk_weights, extras.live_rows,
                             nullptr, p.top_k, p.M, p.K, p.N, p.E, p.sorted_num, p.bpc};
-    if ((phases & 2) && dual) {
+    if ((phases & 2) && dec.dual) {
         Args up = a;
         up.zero_out = extras.out_rows ? 0 : 1;
         up.pregathered = a_mode;
@@ -1903,7 +1908,7 @@ int run(const Problem &p, void *workspace, size_t workspace_bytes, cudaStream_t 
         cfg.numAttrs = up.use_pdl ? 1 : 0;
         PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, up_kernel, map_x, map_w1, map_act, map_x_short, map_act_short, up));
     }
-    if ((phases & 4) && token_n_down) return run_tokn_bf16(tdown, workspace, nullptr, ws_base + lay.items, 4, stream);
+    if ((phases & 4) && dec.token_n_down) return run_tokn_bf16(tdown, workspace, nullptr, ws_base + lay.items, 4, stream);
     if (phases & 4) {
         Args dn = a;
         dn.use_pdl = (pdl_enabled() && (phases & 2)) ? 1 : 0;
@@ -1963,8 +1968,20 @@ extern "C" size_t pmoe_debug_bf16_workspace_extent(int M, int K, int N, int num_
     size_t end = rows * (N / 2) * 2;                                  // activation
     if (d.pregather) end = std::max(end, lay.x_sorted + rows * K * 2);
     if (d.tails) end = std::max(end, lay.lists + (2 * (rows / 256) + 2) * sizeof(int32_t));
-    if (d.token_n || (bpc == 1 && token_n_enabled())) end = std::max(end, lay.items + tokn_items_bytes(sorted_num));
+    if (d.token_n || d.token_n_down) end = std::max(end, lay.items + tokn_items_bytes(sorted_num));
     return end;
+}
+
+extern "C" int pmoe_debug_bf16_route(int M, int K, int N, int num_experts, int top_k, int bpc, int with_live_rows) {
+    using namespace pmoe;
+    static const int32_t some = 0;
+    Problem p{};
+    p.M = M, p.K = K, p.N = N, p.E = num_experts, p.top_k = top_k, p.bpc = bpc, p.split = 1;
+    call_extras().live_rows = with_live_rows ? &some : nullptr;   // not read
+    const Decisions d = decide(p);
+    call_extras() = CallExtras{};
+    return (d.token_n ? PMOE_ROUTE_TOKEN_N_UP | PMOE_ROUTE_TOKEN_N_DOWN : 0) | (d.dual ? PMOE_ROUTE_TWO_BLOCK_UP : 0) |
+           (d.token_n_down ? PMOE_ROUTE_TOKEN_N_DOWN : 0) | (bpc == 2 && !d.token_n ? PMOE_ROUTE_CTA_PAIRS : 0);
 }
 
 extern "C" int pmoe_fused_moe_bf16_ws(const void *x, const void *w, const void *w2, void *out,

@@ -96,6 +96,31 @@ def test_bf16_workspace_covers_every_launch_path(lib, monkeypatch, pregather, ag
                 assert size >= sorted_num * (N // 2 + K) * 2 + (sorted_num // 128 + 2) * 4
 
 
+TOKEN_N, TOKEN_N_DOWN, TWO_BLOCK_UP, CTA_PAIRS = 3, 2, 4, 8
+
+
+@pytest.mark.parametrize("M,K,N,E,k,bpc,live,route", [
+    (8192, 2048, 1536, 128, 8, 1, False, TOKEN_N),
+    (4096, 4096, 28672, 8, 2, 2, False, TOKEN_N),
+    (65536, 4096, 3072, 128, 8, 1, False, TWO_BLOCK_UP + TOKEN_N_DOWN),
+    (9600, 2048, 768, 128, 8, 1, False, 0),
+    # long rows on narrow layers: the token-N down kernel only where its saving covers the launch for its work items
+    (4400, 5120, 2048, 16, 4, 1, False, TWO_BLOCK_UP + TOKEN_N_DOWN),
+    (4400, 5120, 1792, 16, 4, 1, False, TWO_BLOCK_UP),
+    (4400, 2560, 1280, 16, 4, 1, False, TWO_BLOCK_UP),
+    # M is a capacity: the rows in use are not known here
+    (8192, 4096, 3072, 16, 8, 1, True, TWO_BLOCK_UP),
+    (8192, 4096, 3072, 16, 8, 1, False, TWO_BLOCK_UP + TOKEN_N_DOWN),
+    (1024, 4096, 3072, 16, 8, 1, True, TOKEN_N),
+])
+def test_bf16_route(lib, monkeypatch, M, K, N, E, k, bpc, live, route):
+    for name in ("PMOE_TOKN", "PMOE_AGATHER", "PMOE_PREGATHER", "PMOE_DUAL", "PMOE_DOWN_BULK", "PMOE_PAIR_TAILS", "PMOE_SHORT_A"):
+        monkeypatch.delenv(name, raising=False)
+    assert lib.pmoe_debug_bf16_route(M, K, N, E, k, bpc, int(live)) == route
+    monkeypatch.setenv("PMOE_TOKN", "0")
+    assert lib.pmoe_debug_bf16_route(M, K, N, E, k, bpc, int(live)) & TOKEN_N == 0
+
+
 def test_bf16_ws_entry_point_rejects_a_short_workspace(lib):
     """The `_ws` entry point checks the caller's size against the full layout before any launch."""
     buf = (C.c_char * 8192)()
