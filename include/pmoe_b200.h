@@ -58,7 +58,8 @@ int pmoe_version(void);
  * `pmoe_moe_align` takes its scratch from the stream-ordered allocator (cudaMallocAsync);
  * `pmoe_moe_align_ws` uses caller memory of at least `pmoe_moe_align_workspace_bytes` bytes (up to 4096 ids, or 16384
  * with at most 256 experts, may come without: one CTA then aligns them, more slowly)
- * (may be 0 for small n), 16-byte aligned, and performs no allocation. */
+ * (may be 0 for small n), 16-byte aligned, and performs no allocation. Scratch sized for the largest n serves every
+ * smaller one. */
 int pmoe_moe_align(const int32_t *topk_ids, int32_t *sorted_token_ids, int32_t *expert_ids,
                    int32_t *num_tokens_post_padded, int n, int num_experts, int block_m, int pad_to,
                    int max_padded, int max_blocks, pmoe_stream_t stream);

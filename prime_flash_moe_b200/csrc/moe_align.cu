@@ -309,12 +309,13 @@ struct Plan {
 constexpr int kIdsPerCtaMin = 2048;        // every CTA reads the counters of all: few large segments ...
 constexpr int kIdsPerCtaMinShort = 512;    // ... but not so few that a short problem leaves the chip idle
 
-Plan make_plan(int n, int E) {
+Plan make_plan(int n, int E, size_t max_ctas = static_cast<size_t>(-1)) {
     Plan p{};
     if (n <= kOneCtaN) return p;
     const int per_cta = n <= kSmallN32 ? kIdsPerCtaMinShort : kIdsPerCtaMin;
     int ctas = (n + per_cta - 1) / per_cta;
     ctas = std::max(1, std::min(ctas, sm_count()));
+    ctas = static_cast<int>(std::min<size_t>(ctas, max_ctas));
     p.ctas = ctas;
     const int warps = ctas * kWarpsPerCta;
     p.seg = ((n + warps - 1) / warps + 31) & ~31;
@@ -322,12 +323,15 @@ Plan make_plan(int n, int E) {
     return p;
 }
 
-// the plan of a call whose scratch may be missing or short: short problems then run on one CTA
+// The plan of a call whose scratch may be missing or short: short problems then run on one CTA, others on as many as the
+// scratch holds counters for, down to one per kIdsPerCtaMin ids. (What a problem can use does not grow with n: 16384 ids
+// take 32 CTAs, 16385 nine. Scratch allocated for the largest n a program meets thus serves every smaller one.)
 Plan plan_with_scratch(int n, int E, const void *workspace, size_t workspace_bytes) {
     const Plan p = make_plan(n, E);
-    if ((!workspace || workspace_bytes < p.ws_ints * sizeof(int)) && (n <= kSmallN || (n <= kSmallN32 && E <= 256)))
-        return Plan{};
-    return p;
+    const size_t fit = workspace ? workspace_bytes / (static_cast<size_t>(E) * sizeof(int)) : 0;
+    if (fit >= static_cast<size_t>(p.ctas)) return p;
+    if (n <= kSmallN || (n <= kSmallN32 && E <= 256)) return Plan{};
+    return fit >= static_cast<size_t>((n + kIdsPerCtaMin - 1) / kIdsPerCtaMin) ? make_plan(n, E, fit) : p;
 }
 
 int check_args(const void *topk_ids, const void *sorted, const void *expert_ids, const void *npp, int n, int E,

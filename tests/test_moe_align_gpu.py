@@ -108,3 +108,26 @@ def test_equals_reference_kernel(T, E, k, bpc, dist):
     assert np.array_equal(mine[1], re_)
     assert np.array_equal(O.canonical_alignment(mine[0], mine[1], mine[2], 128),
                           O.canonical_alignment(rs, re_, rn, 128))
+
+
+@pytest.mark.parametrize("E", [128, 300, 1024])
+@pytest.mark.parametrize("largest", [17000, 40000])
+def test_scratch_of_the_largest_call_serves_the_smaller_ones(E, largest):
+    """Scratch as `pmoe_moe_align_workspace_bytes` reports it for the largest n; less than one CTA's counters per 2048
+    ids is refused."""
+    from prime_flash_moe_b200 import capi
+    lib = capi.lib()
+    scratch = torch.empty(lib.pmoe_moe_align_workspace_bytes(largest, E), dtype=torch.uint8, device="cuda")
+    for n in (2049, 4096, 4097, 8192, 8193, 16384, 16385, largest):
+        ids = torch.randint(0, E, (n, 1), dtype=torch.int32, generator=torch.Generator().manual_seed(n))
+        dev = ids.cuda()
+        max_padded = (n + E * 127 + 127) // 128 * 128
+        out = [torch.empty(m, dtype=torch.int32, device="cuda") for m in (max_padded, max_padded // 128, 1)]
+        args = (dev.data_ptr(), *(t.data_ptr() for t in out), n, E, 128, 128, max_padded, max_padded // 128)
+        st = torch.cuda.current_stream().cuda_stream
+        assert lib.pmoe_moe_align_ws(*args, scratch.data_ptr(), scratch.numel(), st) == 0, (n, lib.pmoe_last_error())
+        for got, ref in zip(out, O.moe_align_spec(ids.numpy(), E, 128, 1)):
+            assert np.array_equal(got.cpu().numpy(), ref), n
+        least = (n + 2047) // 2048 * E * 4
+        one_cta = n <= 4096 or (n <= 16384 and E <= 256)
+        assert lib.pmoe_moe_align_ws(*args, scratch.data_ptr(), least - 4, st) == (0 if one_cta else 1), n
