@@ -307,12 +307,16 @@ struct Plan {
 };
 
 constexpr int kIdsPerCtaMin = 2048;        // every CTA reads the counters of all: few large segments ...
-constexpr int kIdsPerCtaMinShort = 512;    // ... but not so few that a short problem leaves the chip idle
+// ... but not so few that a short problem leaves the chip idle: up to 16384 ids, or 8192 with more than 256 experts, whose
+// counters every CTA sums (us with a CTA per 2048 / 512 ids: 16384 ids, E = 512 17.3 / 19.4, E = 1024 23.4 / 30.5; 8192
+// ids, E = 300 17.4 / 15.4, E = 1024 21.5 / 21.4)
+constexpr int kIdsPerCtaMinShort = 512;
+constexpr int kShortN = 16384, kShortNManyExperts = 8192;
 
 Plan make_plan(int n, int E, size_t max_ctas = static_cast<size_t>(-1)) {
     Plan p{};
     if (n <= kOneCtaN) return p;
-    const int per_cta = n <= kSmallN32 ? kIdsPerCtaMinShort : kIdsPerCtaMin;
+    const int per_cta = n <= (E <= 256 ? kShortN : kShortNManyExperts) ? kIdsPerCtaMinShort : kIdsPerCtaMin;
     int ctas = (n + per_cta - 1) / per_cta;
     ctas = std::max(1, std::min(ctas, sm_count()));
     ctas = static_cast<int>(std::min<size_t>(ctas, max_ctas));
@@ -325,7 +329,7 @@ Plan make_plan(int n, int E, size_t max_ctas = static_cast<size_t>(-1)) {
 
 // The plan of a call whose scratch may be missing or short: short problems then run on one CTA, others on as many as the
 // scratch holds counters for, down to one per kIdsPerCtaMin ids. (What a problem can use does not grow with n: 16384 ids
-// take 32 CTAs, 16385 nine. Scratch allocated for the largest n a program meets thus serves every smaller one.)
+// take 32 CTAs with 256 experts, 16385 nine. Scratch allocated for the largest n a program meets thus serves every smaller one.)
 Plan plan_with_scratch(int n, int E, const void *workspace, size_t workspace_bytes) {
     const Plan p = make_plan(n, E);
     const size_t fit = workspace ? workspace_bytes / (static_cast<size_t>(E) * sizeof(int)) : 0;

@@ -40,6 +40,10 @@ def test_moe_align_argument_errors(lib):
     assert lib.pmoe_moe_align(p, p, p, p, 4, 8, 128, 100, 1024, 8, None) == 1            # pad_to % block_m
     assert lib.pmoe_moe_align_workspace_bytes(1024, 128) == 0                            # single-CTA path
     assert lib.pmoe_moe_align_workspace_bytes(1 << 19, 128) > 0
+    # one row of counters per CTA: a CTA per 512 ids for short problems, per 2048 for the others
+    for n, E, ctas in ((2048, 256, 0), (2049, 256, 5), (16384, 256, 32), (16385, 256, 9), (8192, 257, 16), (8193, 257, 5),
+                       (16384, 1024, 8)):
+        assert lib.pmoe_moe_align_workspace_bytes(n, E) == 4 * E * ctas
 
 
 def _bf16_call(lib, **kw):
