@@ -62,6 +62,7 @@ SIGNATURES = {
     "pmoe_debug_wait_probe": (_i, [_vp]),
     "pmoe_debug_bf16_workspace_extent": (_sz, [_i] * 8),
     "pmoe_debug_bf16_route": (_i, [_i] * 7),
+    "pmoe_debug_backward_route": (_i, [_i] * 5),
 }
 
 _lib = None

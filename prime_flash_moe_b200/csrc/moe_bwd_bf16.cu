@@ -844,10 +844,24 @@ int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, const GArgs &g, cu
 // forward together, us, without / with: 204 rows 1514 / 1604, 313 rows 2371 / 2685, 536 rows 613 / 608, 835 rows 1493 /
 // 1434, 1131 rows 602 / 492). Row space: only for wide layers from 1024 rows on, where the launch for the experts' odd
 // last blocks is small beside the pairs (N = 28672: recompute 1643 -> 1264 + 196, d_act 973 -> 777 + 124, d_xs 1709 ->
-// 1256 + 239; 764 rows 4491 / 4625).
+// 1256 + 239; 764 rows 4491 / 4625), and from three rounds of tiles in the narrowest of the three GEMMs: with fewer the
+// rounding of the pairs' rounds and of the single blocks' launch costs more (whole backward pass with pairs / without, 196
+// random layers of 1 to 11 experts: below one round 0.92 - 1.41, one to two 0.90 - 1.20, two to three 0.88 - 1.09, above
+// 0.85 - 1.03).
 int pairs_mode() {
     const char *v = getenv("PMOE_BWD_PAIRS");
     return (v && v[0] >= '0' && v[0] <= '2') ? v[0] - '0' : -1;
+}
+
+struct BwdRoute {
+    bool wgrad_pairs, row_pairs;
+};
+BwdRoute bwd_route(int T, int K, int N, int E, int top_k) {
+    const int pm = pairs_mode();
+    if (pm >= 0) return {pm >= 1, pm == 2};
+    const long long routed = static_cast<long long>(T) * top_k;
+    const bool rounds = routed / 256 * (std::min(K, N / 2) / 256) * 2 >= 3ll * sm_count();
+    return {routed >= 512ll * E, N >= 8192 && routed >= 1024ll * E && rounds};
 }
 
 template <int MODE>
@@ -926,6 +940,11 @@ extern "C" int pmoe_debug_set_backward_mask(int mask) {
     return old;
 }
 
+extern "C" int pmoe_debug_backward_route(int T, int K, int N, int num_experts, int top_k) {
+    const pmoe::BwdRoute r = pmoe::bwd_route(T, K, N, num_experts, top_k);
+    return (r.wgrad_pairs ? 1 : 0) | (r.row_pairs ? 2 : 0);
+}
+
 extern "C" size_t pmoe_fused_moe_bf16_backward_workspace_bytes(int T, int K, int N, int num_experts, int top_k,
                                                                int sorted_num) {
     if (T <= 0 || K <= 0 || N <= 0 || num_experts <= 0 || top_k <= 0 || sorted_num <= 0) return 0;
@@ -996,10 +1015,8 @@ extern "C" int pmoe_fused_moe_bf16_backward_ex(const void *x, const void *w1, co
     const uint64_t R = static_cast<uint64_t>(sorted_num);
 
     const int mask = g_bwd_mask;
-    const int pm = pairs_mode();
-    const long long routed = static_cast<long long>(T) * top_k;
-    const bool pairs = pm >= 0 ? pm >= 1 : routed >= 512ll * E;                            // weight gradients
-    const bool row_pairs = pm >= 0 ? pm == 2 : N >= 8192 && routed >= 1024ll * E;
+    const BwdRoute route = bwd_route(T, K, N, E, top_k);
+    const bool pairs = route.wgrad_pairs, row_pairs = route.row_pairs;
     const int copy_grid = 8 * sm_count();
     if (mask & 1) {
         PMOE_CUDA_OK(cudaMemsetAsync(inv, 0xFF, static_cast<size_t>(T) * top_k * sizeof(int32_t), stream));

@@ -59,6 +59,30 @@ def test_cta_pair_settings_agree_with_the_oracle(pairs, monkeypatch):
     check(run_backward(x, w1, w2, ids, wts, d_out), refs)
 
 
+@pytest.mark.parametrize("K,N", [(1152, 8320), (1344, 8192)])       # ragged in every GEMM: K, H and N not multiples of 256
+def test_default_row_space_pairs_on_odd_shapes(K, N, monkeypatch):
+    """The layers that take CTA pairs for the row-space GEMMs by default, against the one-CTA kernels (which the cases
+    above compare with the oracle): experts with odd and even block counts, one with a single row, one without any."""
+    from prime_flash_moe_b200 import capi
+    monkeypatch.delenv("PMOE_BWD_PAIRS", raising=False)
+    counts = [5000, 1, 0, 4481, 3300, 4096]
+    E, T = len(counts), sum(counts)
+    assert capi.lib().pmoe_debug_backward_route(T, K, N, E, 1) == 3
+    g = torch.Generator(device=DEV).manual_seed(K)
+    ids = torch.cat([torch.full((c,), e, dtype=torch.int32, device=DEV) for e, c in enumerate(counts)])
+    ids = ids[torch.randperm(T, generator=g, device=DEV)].view(T, 1).contiguous()
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device=DEV, dtype=torch.bfloat16)
+    x, d_out, wts = rnd(T, K), rnd(T, K), torch.rand(T, 1, generator=g, device=DEV) + 0.5
+    w1, w2 = rnd(E, N, K) * K ** -0.5, rnd(E, K, N // 2) * (N // 2) ** -0.5
+    s, e, n = capi.moe_align(ids, E, 128, 1)
+    pairs = capi.fused_moe_bf16_backward(x, w1, w2, d_out, s, e, n, wts, 1)
+    monkeypatch.setenv("PMOE_BWD_PAIRS", "0")
+    single = capi.fused_moe_bf16_backward(x, w1, w2, d_out, s, e, n, wts, 1)
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    check(tuple(t.cpu() for t in pairs), tuple(t.float().cpu() for t in single))
+
+
 @pytest.mark.parametrize("pairs", ["0", "1"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_weight_gradients_in_fp32_and_accumulated(dtype, pairs, monkeypatch):

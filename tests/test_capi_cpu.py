@@ -162,6 +162,23 @@ def test_backward_argument_errors_and_workspace_plan(lib):
     assert lib.pmoe_debug_set_backward_mask(127) == 127
 
 
+@pytest.mark.parametrize("T,K,N,E,k,route", [
+    (4096, 4096, 28672, 8, 2, 3),
+    (4095, 4096, 28672, 8, 2, 1),        # just under 1024 rows per expert
+    (1130, 1280, 19456, 1, 1, 1),        # a third of a round of tiles in d_xs
+    (6400, 1152, 8192, 4, 2, 1),         # 2.7 rounds
+    (8000, 1152, 8192, 4, 2, 3),
+    (8192, 2048, 1536, 128, 8, 1),
+    (4099, 2048, 1536, 128, 8, 0),
+])
+def test_backward_route(lib, monkeypatch, T, K, N, E, k, route):
+    monkeypatch.delenv("PMOE_BWD_PAIRS", raising=False)
+    assert lib.pmoe_debug_backward_route(T, K, N, E, k) == route
+    for mode, forced in (("0", 0), ("1", 1), ("2", 3)):
+        monkeypatch.setenv("PMOE_BWD_PAIRS", mode)
+        assert lib.pmoe_debug_backward_route(T, K, N, E, k) == forced
+
+
 def test_wait_limit_argument_range(lib):
     assert lib.pmoe_debug_set_wait_ns(10) == 1                   # below 1 microsecond
     assert lib.pmoe_debug_set_wait_ns(10 ** 12) == 1             # above 60 seconds
