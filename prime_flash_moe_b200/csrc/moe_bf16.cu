@@ -1589,7 +1589,8 @@ Decisions decide(const Problem &p) {
     // N = 1024, 2813 rows 3160 / 4080; but N = 1536, 512 rows 801 / 724)
     // A batch whose gate/up tiles fill the SMs once but not the CTA pairs (each pair would take a second, mostly empty
     // round) is left to the row-M kernels too when K is long (10 experts x 12 tiles, K = 3456: 67 / 70 us, but 18 x 8,
-    // K = 2176: 59 / 57; 5 x 25, K = 1408: 59 / 51).
+    // K = 2176: 59 / 57; 5 x 25, K = 1408: 59 / 51; with several row blocks an expert 8 experts, 309 rows each, K = 5376,
+    // N = 1536 97 / 107, 2, 373, K = 6656, N = 5376 106 / 122).
     // A narrow layer whose tiles fit one round of the CTA pairs is faster on the token-N kernels all the same: they split
     // the long gate/up contraction's weights over two SMs (9 experts, K = 4992, N = 1024, 50 rows each: 70 / 57 us; 8
     // experts, K = 4864, N = 512, 168 rows: 68 / 60; above one round 22 experts, N = 1024, 83 rows: 89 / 95).
@@ -1598,12 +1599,25 @@ Decisions decide(const Problem &p) {
     // the layer's width (row-M / token-N: K = 4096, N = 3072, 524288 Zipf rows 18.8 / 20.0 ms at the cap, though 18.1 /
     // 16.7 ms on a cool chip; K = 2688, N = 1280 1916 / 2010 us; but K = 2304, N = 2816 4294 / 3878 us; K = 5248, N = 5120
     // 2428 / 1961; K = 2176, N = 2048 319 / 282).
+    // Where the row-M gate/up tiles of up to 1024 rows per expert fill one round of the SMs, each with as many MMAs as a
+    // tile of a CTA pair, the row copy and the planning are all that the token-N kernels add, unless K is long (row-M /
+    // token-N, us: 5 experts, 958 rows each, K = 1536, N = 768 38 / 48; 4, 800, K = 1408, N = 512 34 / 42; 6, 477, K = 2304,
+    // N = 1024 44 / 52; 3, 379, K = 3200, N = 512 40 / 44; but 3, 260, K = 4608, N = 2304 109 / 97; 4, 168, K = 5376,
+    // N = 1024 85 / 75; 1, 337, K = 4864, N = 6912 113 / 98). Of 400 + 400 + 400 random shapes this rule takes 59 to the
+    // row-M kernels, three of which were 3 to 5 % faster on the others.
     const long long rows = static_cast<long long>(p.M) * p.top_k, experts = std::min<long long>(p.E, rows);
-    const long long tiles = experts * (p.N / 256);
-    const bool second_round = 2 * tiles > sm_count() && tiles <= sm_count() && p.K >= 3072;
+    const long long per = rows / p.E, blocks = experts * std::max(1ll, (per + 127) / 128);
+    const long long tiles = experts * (p.N / 256), pair_tiles = experts * std::max(1ll, (per + 255) / 256) * (p.N / 256);
+    const bool row_m_round = p.bpc == 1 && blocks * (p.N / 256) <= sm_count() && per < 1024;
+    const bool second_round = p.K >= 3072 && ((2 * tiles > sm_count() && tiles <= sm_count()) ||
+                                              (2 * pair_tiles > sm_count() && row_m_round));
     const bool one_round = 2 * (experts + rows / 256) * (p.N / 256) <= sm_count();
+    const bool short_round = row_m_round && p.N <= 2048 && per >= 200 && 12 * per >= p.K;
+    // (N = 1280 counts as narrow from 500 to 1023 rows per expert: of 17 random shapes there none gains on the token-N
+    // kernels, mean +7 %; 86 experts, 844 rows each, K = 4096 1078 / 1219 us)
+    const bool wide = p.N > (per >= 500 && per < 1024 ? 1280 : 1024) && (8ll * p.K <= 9ll * p.N || rows < 1024ll * p.E);
     d.token_n = token_n_enabled() && !call_extras().out_rows &&
-                ((p.N > 1024 && !second_round && (8ll * p.K <= 9ll * p.N || rows < 1024ll * p.E)) || one_round || token_n_forced());
+                (token_n_forced() || (!short_round && ((wide && !second_round) || one_round)));
     // PMOE_DUAL=0/1, unset = two blocks for calls with >= 1024 routed rows per expert on average (measured: gate/up
     // kernel -4..-5 % there with the in-kernel gather, -13..-15 % when fed by TMA from the row-gathered copy; +5 % at 512
     // rows per expert, where more pairs straddle two experts)

@@ -112,6 +112,19 @@ TOKEN_N, TOKEN_N_DOWN, TWO_BLOCK_UP, CTA_PAIRS = 3, 2, 4, 8
     (4400, 5120, 2048, 16, 4, 1, False, TWO_BLOCK_UP + TOKEN_N_DOWN),
     (4400, 5120, 1792, 16, 4, 1, False, TWO_BLOCK_UP),
     (4400, 2560, 1280, 16, 4, 1, False, TWO_BLOCK_UP),
+    # one round of row-M tiles with 200 to 1023 rows per expert and a short K
+    (2395, 1536, 768, 5, 2, 1, False, 0),
+    (1600, 1408, 512, 4, 2, 1, False, 0),
+    (1600, 1408, 512, 4, 2, 2, False, TOKEN_N),
+    (954, 2304, 1024, 6, 3, 1, False, 0),
+    (391, 4608, 2304, 3, 2, 1, False, TOKEN_N),
+    (336, 4864, 512, 8, 4, 1, False, TOKEN_N),
+    (256, 4096, 512, 8, 4, 1, False, TOKEN_N),
+    (10000, 4096, 1280, 40, 2, 1, False, 0),
+    (9800, 4096, 1280, 40, 2, 1, False, TOKEN_N),
+    (10000, 4096, 1536, 40, 2, 1, False, TOKEN_N),
+    # one round of row-M tiles but two of the CTA pairs
+    (412, 5376, 1536, 8, 6, 1, False, 0),
     # M is a capacity: the rows in use are not known here
     (8192, 4096, 3072, 16, 8, 1, True, TWO_BLOCK_UP),
     (8192, 4096, 3072, 16, 8, 1, False, TWO_BLOCK_UP + TOKEN_N_DOWN),
