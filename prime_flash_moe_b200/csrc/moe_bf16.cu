@@ -1624,11 +1624,13 @@ Decisions decide(const Problem &p) {
     const int dual_env = dual_blocks_mode();
     d.dual = p.bpc == 1 && !d.token_n && d.a_mode != 0 && (dual_env < 0 ? rows >= 1024ll * p.E : dual_env != 0);
     // The two-block gate/up kernel hands its activations to the token-N down kernel where that saves more than the launch
-    // for its work items costs, about 15 us: on layers of N >= 2048 (whole call, us, without / with: K = 4096, N = 3072,
-    // 524288 rows 18600 / 17700; N = 2560, 16 experts, 1100 rows each, K = 5120 741 / 701; N = 2048, K = 5120 546 / 535;
-    // but N = 1536, K = 2048 177 / 193; N = 1280, K = 2560 195 / 218). Not with live_rows: M is then the capacity of a
-    // buffer of which few rows may be in use (capacity 8192, 32 rows in use, K = 4096, N = 3072: 247 / 265).
-    d.token_n_down = d.dual && p.N >= 2048 && token_n_enabled() && !call_extras().out_rows && !call_extras().live_rows;
+    // for its work items costs, about 15 us. Whole call with / without, N >= 2048, 5500 random shapes by rows * K * N: below
+    // 1.0e11 1.00 - 1.03, to 1.4e11 0.98 - 1.01, to 2.5e11 0.96 - 0.99, to 1e12 0.94 - 0.97; K = 4096, N = 3072, 524288
+    // rows 18600 / 17700 us. Narrower layers lose or gain nothing (N = 1536, K = 2048 177 / 193 us; N = 1280, K = 2560
+    // 195 / 218). Not with live_rows: M is then the capacity of a buffer of which few rows may be in use (capacity 8192, 32
+    // rows in use, K = 4096, N = 3072: 247 / 265).
+    d.token_n_down = d.dual && p.N >= 2048 && rows * p.K >= (1ll << 37) / p.N && token_n_enabled() &&
+                     !call_extras().out_rows && !call_extras().live_rows;
     return d;
 }
 

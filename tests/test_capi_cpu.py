@@ -111,6 +111,7 @@ TOKEN_N, TOKEN_N_DOWN, TWO_BLOCK_UP, CTA_PAIRS = 3, 2, 4, 8
     # long rows on narrow layers: the token-N down kernel only where its saving covers the launch for its work items
     (4400, 5120, 2048, 16, 4, 1, False, TWO_BLOCK_UP + TOKEN_N_DOWN),
     (4400, 5120, 1792, 16, 4, 1, False, TWO_BLOCK_UP),
+    (4400, 2560, 2048, 16, 4, 1, False, TWO_BLOCK_UP),
     (4400, 2560, 1280, 16, 4, 1, False, TWO_BLOCK_UP),
     # one round of row-M tiles with 200 to 1023 rows per expert and a short K
     (2395, 1536, 768, 5, 2, 1, False, 0),
