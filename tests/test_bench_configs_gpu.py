@@ -102,10 +102,14 @@ def test_c1_mixtral_cta_pairs_full_size(monkeypatch):
         assert O.max_rel_to_peak(out[toks].cpu(), ref) <= TOL
 
 
+@pytest.mark.parametrize("token_n", [None, "0", "1"])
 @pytest.mark.parametrize("T", [8192, 16384])
-def test_c2_qwen3_bf16_default_paths(T):
-    """Configuration 2 at T=8192 (in-kernel row gather, one row block per tile) and T=16384 (two row blocks per
-    tile: 1024 routed rows per expert), whatever the launcher picks by default."""
+def test_c2_qwen3_bf16(T, token_n, monkeypatch):
+    """Configuration 2 at T=8192 and T=16384 (1024 routed rows per expert) on the kernels the launcher picks by default
+    (token-N; two row blocks per tile), on the row-M ones (in-kernel row gather with one and with two row blocks per
+    tile) and on the token-N ones."""
+    if token_n is not None:
+        monkeypatch.setenv("PMOE_TOKN", token_n)
     K, E, N, k = 2048, 128, 1536, 8
     x, w1, w2, ids, wts = device_case(T, K, E, N, k, seed=T)
     out = run_bf16(x, w1, w2, ids, wts)

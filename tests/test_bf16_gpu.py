@@ -35,13 +35,18 @@ def run_mine(x, w1, w2, ids, wts, split, stages=4, bn=64, wn=4, via="capi", bpc=
     return out.cpu()
 
 
-@pytest.mark.parametrize("split", [True, False])
+# kernels of the split pipeline: "0" row-M, "1" token-N; split=False has one set only
+KERNELS = [(True, "0"), (True, "1"), (False, "0")]
+
+
+@pytest.mark.parametrize("split,token_n", KERNELS)
 @pytest.mark.parametrize("T,K,E,N,k", [
     (1, 128, 2, 256, 1), (8, 128, 1, 256, 1), (64, 512, 4, 512, 2), (130, 256, 5, 768, 3),
     (256, 4096, 8, 512, 4),      # benchmark configuration 0
     (300, 1024, 8, 1024, 4), (1000, 384, 16, 256, 8),
 ])
-def test_vs_fp32_oracle(T, K, E, N, k, split):
+def test_vs_fp32_oracle(T, K, E, N, k, split, token_n, monkeypatch):
+    monkeypatch.setenv("PMOE_TOKN", token_n)
     x, w1, w2, ids, wts = O.make_case(T, K, E, N, k, seed=T + K)
     ref = O.moe_ref_fp32(x, w1, w2, ids, wts)
     out = run_mine(x, w1, w2, ids, wts, split)
@@ -49,10 +54,12 @@ def test_vs_fp32_oracle(T, K, E, N, k, split):
     assert O.max_rel_to_peak(out, ref) <= TOL
 
 
-@pytest.mark.parametrize("split", [True, False])
+@pytest.mark.parametrize("split,token_n", KERNELS)
 @pytest.mark.parametrize("bn,wn", [(64, 4), (32, 8)])
 @pytest.mark.parametrize("stages", [1, 2, 3, 4, 5])
-def test_knobs(split, bn, wn, stages):
+def test_knobs(split, token_n, bn, wn, stages, monkeypatch):
+    """Every accepted setting gives the same result; the token-N kernels check the knobs and do not use them."""
+    monkeypatch.setenv("PMOE_TOKN", token_n)
     if split and stages == 5:
         pytest.skip("split=True accepts stages <= 4 (checked in test_argument_checks)")
     x, w1, w2, ids, wts = O.make_case(200, 512, 6, 512, 3, seed=stages)
@@ -296,13 +303,15 @@ def test_dual_block_tiles(T, K, E, N, k, bn, wn, stages, agather, monkeypatch):
     assert O.max_rel_to_peak(dual, one.float()) <= TOL
 
 
+@pytest.mark.parametrize("token_n", ["0", "1"])
 @pytest.mark.parametrize("bpc", [1, 2])
-def test_ex_entry_point_live_rows_and_output_addresses(bpc):
+def test_ex_entry_point_live_rows_and_output_addresses(bpc, token_n, monkeypatch):
     """`pmoe_fused_moe_bf16_ex` (the expert-parallel mode's entry point). live_rows: buffers sized for a worst case,
     only the leading rows in use - the library zeroes just those rows of `out`. out_rows: every output row has its
     own address (here rows of a second buffer in permuted order; across GPUs: rows of the source rank's buffer) and
     the down kernels ADD their results there, zeroing nothing."""
     from prime_flash_moe_b200 import capi
+    monkeypatch.setenv("PMOE_TOKN", token_n)
     T, cap, K, E, N, k = 300, 512, 512, 4, 512, 2
     x, w1, w2, ids, wts = O.make_case(T, K, E, N, k, seed=77)
     ref = O.moe_ref_fp32(x, w1, w2, ids, wts)

@@ -160,14 +160,20 @@ def test_argument_checks():
                                      workspace=small[(-small.data_ptr()) % 1024:][:1024])
 
 
-@pytest.mark.parametrize("bpc", [1, 2])
+TOKEN_N, TWO_BLOCK_UP, CTA_PAIRS = 3, 4, 8      # pmoe_debug_bf16_route
+
+
+@pytest.mark.parametrize("bpc,token_n", [(1, "0"), (2, "0"), (1, "1"), (2, "1")])
 @pytest.mark.parametrize("T,K,E,N,k", [(64, 512, 4, 512, 2), (256, 4096, 8, 512, 4), (2100, 256, 2, 768, 1)])
-def test_kept_pre_activations(T, K, E, N, k, bpc):
+def test_kept_pre_activations(T, K, E, N, k, bpc, token_n, monkeypatch):
     """The forward call that keeps gate | up: same `out` as the plain call, the kept rows equal xs @ W1[e]^T, and the
-    backward pass fed with them matches the oracle (the last shape has > 1024 rows per expert: the two-block
-    gate/up kernel). bpc = 2: routing tables padded to 256 rows, CTA-pair gate/up kernel + single-block tails, and
-    a backward pass that skips the blocks without routed rows."""
+    backward pass fed with them matches the oracle. Row-M kernels: one row block per tile, two (the last shape has > 1024
+    rows per expert), CTA pairs + single-block tails (bpc = 2: routing tables padded to 256 rows, and a backward pass
+    that skips the blocks without routed rows); and the token-N kernels on the same tables."""
+    monkeypatch.setenv("PMOE_TOKN", token_n)
+    route = TOKEN_N if token_n == "1" else CTA_PAIRS if bpc == 2 else TWO_BLOCK_UP if T * k >= 1024 * E else 0
     from prime_flash_moe_b200 import capi
+    assert capi.lib().pmoe_debug_bf16_route(T, K, N, E, k, bpc, 0) == route
     x, w1, w2, ids, wts = O.make_case(T, K, E, N, k, seed=T + 3)
     d_out = torch.randn(T, K, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16)
     s, e, n = capi.moe_align(ids.to(DEV), E, 128, bpc)
@@ -187,6 +193,35 @@ def test_kept_pre_activations(T, K, E, N, k, bpc):
     torch.cuda.synchronize()
     assert capi.device_status() == 0
     check(tuple(g.cpu() for g in grads), O.moe_backward_ref_fp32(x, w1, w2, ids, wts, d_out))
+
+
+def test_kept_two_block_gate_up_followed_by_the_token_n_down_kernel(monkeypatch):
+    """Long rows on a layer with 8 K > 9 N: by default the two-block gate/up kernel and the token-N down kernel. Against
+    the row-M kernels: `out`, the kept rows and the gradients."""
+    from prime_flash_moe_b200 import capi
+    monkeypatch.delenv("PMOE_TOKN", raising=False)
+    counts = [5000, 5, 0, 3611, 4670]
+    K, N, E, T = 4608, 2304, len(counts), sum(counts)
+    assert capi.lib().pmoe_debug_bf16_route(T, K, N, E, 1, 1, 0) == TWO_BLOCK_UP + 2
+    g = torch.Generator(device=DEV).manual_seed(1)
+    ids = torch.cat([torch.full((c,), e, dtype=torch.int32, device=DEV) for e, c in enumerate(counts)])
+    ids = ids[torch.randperm(T, generator=g, device=DEV)].view(T, 1).contiguous()
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device=DEV, dtype=torch.bfloat16)
+    x, d_out, wts = rnd(T, K), rnd(T, K), torch.rand(T, 1, generator=g, device=DEV) + 0.5
+    w1, w2 = rnd(E, N, K) * K ** -0.5, rnd(E, K, N // 2) * (N // 2) ** -0.5
+    s, e, n = capi.moe_align(ids, E, 128, 1)
+    results = []
+    for token_n in (None, "0"):
+        if token_n:
+            monkeypatch.setenv("PMOE_TOKN", token_n)
+        out, gate_up = capi.fused_moe_bf16_keep(x, w1, w2, s, e, n, wts, torch.full_like(x, float("nan")), 1)
+        grads = capi.fused_moe_bf16_backward(x, w1, w2, d_out, s, e, n, wts, 1, gate_up=gate_up)
+        results.append((out, gate_up[s >= 0], *grads))
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    for got, ref in zip(*results):
+        assert torch.isfinite(got.float()).all()
+        assert O.max_rel_to_peak(got, ref) <= 1e-2        # bf16 results, fp32 sums in another order
 
 
 @pytest.mark.parametrize("fill", [float("nan"), float("inf")])

@@ -151,17 +151,26 @@ def test_route_then_align_then_moe():
 
 @pytest.mark.parametrize("via", ["capi", "torch"])
 @pytest.mark.parametrize("T,E,k,bpc,dtype", [
-    (64, 8, 2, 1, torch.float32),            # one CTA aligns it: router kernel + small align kernel
-    (4096, 8, 2, 2, torch.float32),          # n = 8192, E <= 256: still one CTA
-    (8192, 128, 8, 1, torch.float32),        # fused router + histogram kernel, then the scatter pass
+    (64, 8, 2, 1, torch.float32),            # router kernel + one align CTA
+    (4096, 8, 2, 2, torch.float32),          # n = 8192: sixteen align CTAs
+    (8192, 128, 8, 1, torch.float32),
     (16384, 256, 8, 1, torch.bfloat16),
     (20000, 64, 4, 2, torch.float32),
-    (9000, 100, 5, 1, torch.float32),        # top_k = 5 does not divide a CTA's id range: the separate kernels
+    (9000, 100, 5, 1, torch.float32),
     (3000, 1024, 8, 1, torch.float32),
+    (2048, 16, 1, 1, torch.float32), (2049, 16, 1, 2, torch.float32),        # one / several align CTAs
+    (16384, 16, 1, 1, torch.float32), (16385, 16, 1, 1, torch.float32),      # a CTA per 512 / per 2048 ids
+    (8192, 300, 1, 1, torch.float32), (8193, 300, 1, 1, torch.float32),      # the same with more than 256 experts
+    # one launch routes and aligns up to 32 tokens (32 warps), or 8 with more than 256 experts (8 warps)
+    *[(T, E, k, bpc, dtype) for T in (1, 31, 32, 33) for E, k, bpc, dtype in (
+        (8, 2, 1, torch.float32), (40, 32, 2, torch.bfloat16), (128, 8, 2, torch.float32), (256, 32, 1, torch.bfloat16))],
+    *[(T, E, k, bpc, dtype) for T in (1, 8, 9) for E, k, bpc, dtype in (
+        (257, 8, 1, torch.float32), (512, 32, 2, torch.bfloat16), (768, 8, 2, torch.float32), (769, 32, 1, torch.bfloat16),
+        (1024, 8, 1, torch.float32))],
 ])
 def test_route_topk_align_equals_the_two_separate_calls(T, E, k, bpc, dtype, via):
-    """Router fused with the moe_align histogram pass: all five outputs identical, bit for bit, to route_topk
-    followed by moe_align on its ids - and the routing tables to the CPU restatement of the reference's."""
+    """Router and moe_align in one call: all five outputs identical, bit for bit, to route_topk followed by moe_align on
+    its ids - and the routing tables to the CPU restatement of the reference's."""
     import numpy as np
     import prime_flash_moe_b200 as P
     from prime_flash_moe_b200 import capi
