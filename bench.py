@@ -352,6 +352,29 @@ def time_calls(call, reps, flush_buf=None):
     return sum(a.elapsed_time(b) for a, b in pairs) / reps
 
 
+def bf16_path(lib, T, K, N, E, k, bpc, sorted_num):
+    """The kernels the split bf16 operator takes for a call of this size under the current environment, as its launcher
+    reports them: names of the gate/up and down kernels, launches per call, whether half-empty row-block pairs run in
+    launches of their own, and what runs under every phase mask beside the kernel it names (timed with it)."""
+    route = lib.pmoe_debug_bf16_route(T, K, N, E, k, bpc, 0)
+    token_n_up, token_n_down, two_block, pairs = route & 1, route & 2, route & 4, route & 8
+    if token_n_up:
+        by_token = T * K * 2 >= 64 << 20 and 2 <= k <= 32 and T * k <= sorted_num     # row info, then the gather by token
+        return {"up": "moe_tokn_kernel<up>", "down": "moe_tokn_kernel<down>", "launches": 4 if by_token else 3,
+                "tails": False, "includes": "gather_plan_kernel without the row copy (up, down)"}
+    if pairs:
+        tails = os.environ.get("PMOE_PAIR_TAILS", "1") != "0"
+        return {"up": "moe_pair_bf16_kernel<up>", "down": "moe_pair_bf16_kernel<down>", "launches": 6 if tails else 3,
+                "tails": tails, "includes": None}
+    pre_pass = {"tma4": False, "pre": True, "lsu": False}.get(os.environ.get("PMOE_AGATHER", ""), N >= 8192 or T * k < 256 * E)
+    if os.environ.get("PMOE_PREGATHER") == "0":
+        pre_pass = False
+    return {"up": "moe_up_dual_bf16_kernel" if two_block else "moe_up_bf16_kernel",
+            "down": "moe_tokn_kernel<down>" if token_n_down else "moe_down_bf16_kernel",
+            "launches": 2 + int(pre_pass) + (1 if token_n_down else 0), "tails": False,
+            "includes": "gather_plan_kernel without the row copy (down)" if token_n_down else None}
+
+
 def weight_streaming_roofline(roof, cfg, ids, per_kernel_up_ms, ms_step, peaks, mx, traffic):
     """Calls with fewer than 256 routed rows per expert are bound by streaming the weights of the experts
     actually routed to, not by the tensor pipe: restate the roofline of the gate/up kernel against the
@@ -506,6 +529,7 @@ def sweep_entry_ours(name, tokens, dtype, device, peaks, stages):
     else:
         call = lambda: capi.fused_moe_bf16(c["x"], c["w1"], c["w2"], s, e, n, c["wts"], out, k, 128, 64, 4, stages, bpc, 1,
                                            True, workspace=ws)
+    path = None if mx else bf16_path(lib, T, K, N, E, k, bpc, s.numel())
     lib.pmoe_debug_set_phase_mask(2)
     up_ms = time_calls(call, 10, flush_buf)
     lib.pmoe_debug_set_phase_mask(4)
@@ -516,8 +540,7 @@ def sweep_entry_ours(name, tokens, dtype, device, peaks, stages):
     assert capi.device_status() == 0, "a kernel recorded an error status"
     wb = (1.0 + 1.0 / 32) if mx else 2.0
     up_bytes = touched * N * K * wb + T * k * K * wb + T * k * (N // 2) * wb + T * K * 2
-    kernel = ("moe_up_mxfp8_kernel" if mx else ("moe_pair_bf16_kernel<up>" if bpc == 2 else "moe_up_bf16_kernel (or its "
-              "two-block variant)"))
+    kernel = "moe_up_mxfp8_kernel" if mx else path["up"]
     if T * k >= 256 * E:       # compute-bound call: tensor roofline of the gate/up kernel
         peak, src = measure_mxfp8_peak(device) if mx else (peaks["bf16_tflops"], peaks["source"] + " (burst cuBLAS bf16)")
         ach = 2.0 * T * k * K * N / (up_ms * 1e-3) / 1e12
@@ -529,6 +552,8 @@ def sweep_entry_ours(name, tokens, dtype, device, peaks, stages):
                 "frac": ach / peaks["hbm_gbs"], "peak_source": peaks["source"] + " (STREAM-style copy)", "traffic": None,
                 "algorithmic_bytes": up_bytes, "experts_touched": touched}
     roof["kernel_ms"] = {"up": up_ms, "down": down_ms}
+    if path:
+        roof.update({"down_kernel": path["down"], "includes": path["includes"]})
     del c, ws, out, flush_buf
     torch.cuda.empty_cache()
     return {"config": name, "tokens": T, "dtype": dtype, "ms_per_step": ms, "value": flops / (ms * 1e-3) / 1e12,
@@ -865,11 +890,12 @@ def run_gpu_arm(args, impl):
         from prime_flash_moe_b200 import capi
         ops = torch.ops.prime_moe
         (bn, wn), stages, split, bpc = ((64, 4) if args.warp_n == 4 else (32, 8)), args.stages, bool(args.split), args.bpc
-        # align kernels + gather, gate/up|fused, down|finalize (+ pair classification and the two tail launches, bpc=2)
-        # moe_align (one CTA up to 4096 ids, or 16384 with <= 256 experts; else histogram + scatter) + row gather,
-        # gate/up|fused, down|finalize (+ pair classification and the two tail launches, bpc=2)
-        align_launches = 1 if (T * k <= 4096 or (T * k <= 16384 and E <= 256)) else 2
-        launches_per_step = align_launches + 3 + (3 if (bpc == 2 and split and not mx) else 0)
+        # moe_align (one CTA when it needs no scratch, else histogram + scatter), then the operator: the split bf16 path as
+        # its launcher reports it; mxfp8 and split=False: row gather, gate/up|fused, down|finalize
+        align_launches = 2 if capi.lib().pmoe_moe_align_workspace_bytes(T * k, E) else 1
+        padded = -(-(T * k + E * (128 * bpc - 1)) // (128 * bpc)) * 128 * bpc
+        op_launches = 3 if (mx or not split) else bf16_path(capi.lib(), T, K, N, E, k, bpc, padded)["launches"]
+        launches_per_step = align_launches + op_launches
 
         def step(x_, ids_, wts_, out_):
             s, e, n = ops.moe_align(ids_, E, 128, bpc)
@@ -987,11 +1013,11 @@ def run_gpu_arm(args, impl):
         call = lambda: capi.fused_moe_bf16(x, w1, w2, s, e, n, wts, out, k, 128, 64 if args.warp_n == 4 else 32, args.warp_n,
                                            args.stages, args.bpc, 1, True, workspace=ws)
         call()
+        path = bf16_path(lib, T, K, N, E, k, args.bpc, s.numel())
         per_kernel = {}
-        masks = [("gather_rows", 1), ("moe_up_bf16", 2), ("moe_down_bf16", 4)]
-        if args.bpc == 2:      # the CTA-pair kernels without the single-block tail launches that follow them
-            masks = [("gather_rows", 1), ("moe_up_bf16", 2 | 8), ("moe_up_bf16_with_tails", 2), ("moe_down_bf16", 4 | 8),
-                     ("moe_down_bf16_with_tails", 4)]
+        masks = [("gather_rows", 1), ("up", 2), ("down", 4)]
+        if path["tails"]:      # the CTA-pair kernels without the single-block tail launches that follow them
+            masks = [("gather_rows", 1), ("up", 2 | 8), ("up_with_tails", 2), ("down", 4 | 8), ("down_with_tails", 4)]
         for name, mask in masks:
             lib.pmoe_debug_set_phase_mask(mask)
             per_kernel[name] = time_calls(call, 20, flush_buf if flush_l2 else None)
@@ -999,25 +1025,27 @@ def run_gpu_arm(args, impl):
         call()
         torch.cuda.synchronize()
         rows_dominant = T * k
-        if args.bpc == 2 and os.environ.get("PMOE_PAIR_TAILS", "1") != "0":
+        if path["tails"]:
             # rows of the half-empty last pairs run on the one-CTA kernels, not on the kernel timed here
             cnt = torch.bincount(ids_cpu.reshape(-1).long(), minlength=E)
             rem = cnt % 256
             rows_dominant -= int(rem[(rem > 0) & (rem <= 128)].sum())
         up_flops = 2.0 * rows_dominant * K * N
-        achieved = up_flops / (per_kernel["moe_up_bf16"] * 1e-3) / 1e12
+        achieved = up_flops / (per_kernel["up"] * 1e-3) / 1e12
         # DRAM bytes of one launch of that kernel, from the ncu captures summarised under profiles/
-        traffic = {("c1", 2): 2.713e9, ("c2", 1): 1.112e9}.get((args.config, args.bpc)) \
-            if (not args.tokens and args.stages == 4 and args.warp_n == 4) else None
-        roofline = {"kernel": "moe_pair_bf16_kernel<up>" if args.bpc == 2 else "moe_up_bf16_kernel", "bound": "tensor",
+        traffic = {("c1", "moe_tokn_kernel<up>"): 4.024e9, ("c1", "moe_pair_bf16_kernel<up>"): 2.713e9,
+                   ("c2", "moe_up_bf16_kernel"): 1.112e9}.get(
+            (args.config, path["up"])) if (not args.tokens and args.stages == 4 and args.warp_n == 4) else None
+        roofline = {"kernel": path["up"], "down_kernel": path["down"], "includes": path["includes"], "bound": "tensor",
                     "rows": rows_dominant, "achieved": achieved,
                     "peak": peaks["bf16_tflops"], "unit": "TFLOP/s", "frac": achieved / peaks["bf16_tflops"],
                     "peak_source": peaks["source"] + " (burst cuBLAS bf16)",
                     "frac_of_sustained": achieved / peaks["bf16_tflops_sustained"] if peaks["bf16_tflops_sustained"] else None,
                     "traffic": traffic, "algorithmic_bytes": float(E * N * K * 2 + rows_dominant * K * 2 + rows_dominant * N + T * K * 2),
                     "kernel_ms": per_kernel, "whole_op_frac": value / world / peaks["bf16_tflops"]}
-        roofline = weight_streaming_roofline(roofline, cfg, ids, per_kernel["moe_up_bf16"], ms_step, peaks, False,
-                                             835.3e6 if (args.config == "c2" and args.tokens == 128) else None)
+        roofline = weight_streaming_roofline(roofline, cfg, ids, per_kernel["up"], ms_step, peaks, False,
+                                             835.3e6 if (args.config == "c2" and args.tokens == 128 and
+                                                         path["up"] == "moe_up_bf16_kernel") else None)
         assert capi.device_status() == 0, "a kernel recorded an error status"
     roof_clocks.__exit__(None, None, None)
     if roofline is not None:
@@ -1104,7 +1132,7 @@ def run_gpu_arm(args, impl):
         # plan (3) + moe_align (1 or 2) + row gather, gate/up, down (3) + combine (1) (+ publish, push, 2 signals,
         # prepare, return: 6 in peer mode)
         n_local = (world * T if layer.combine_mode == "peer" else ep_rows[-1]) * k      # ids moe_align sees on this rank
-        align_launches = 1 if (n_local <= 4096 or (n_local <= 16384 and E // world <= 256)) else 2
+        align_launches = 2 if capi.lib().pmoe_moe_align_workspace_bytes(n_local, E // world) else 1
         launches_per_step = 3 + align_launches + 3 + 1 + (6 if layer.combine_mode == "peer" else 0)
         a_, b_ = out[:np_].float(), par_ref.float()
         ep_parity = max_over_ranks(float((a_ - b_).abs().max() / b_.abs().max().clamp_min(1e-30)), world, device)

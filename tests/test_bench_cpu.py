@@ -65,3 +65,18 @@ def test_sweep_summary_is_one_string_per_entry():
     assert text.count(";") == 2
     assert "c2/T8192/mxfp8: 440us 1400TFLOP/s tensor frac 0.58" in text
     assert "c4/moe_align: 30us 140GB/s hbm frac 0.02" in text and "c3/mxfp8: failed" in text
+
+
+def test_bf16_path_names_the_kernels_the_launcher_takes(monkeypatch):
+    from prime_flash_moe_b200 import capi
+    for name in ("PMOE_TOKN", "PMOE_AGATHER", "PMOE_PREGATHER", "PMOE_DUAL", "PMOE_DOWN_BULK", "PMOE_PAIR_TAILS", "PMOE_SHORT_A"):
+        monkeypatch.delenv(name, raising=False)
+    b = _bench()
+    path = lambda T, K, E, N, k, bpc: tuple(b.bf16_path(capi.lib(), T, K, N, E, k, bpc, T * k + E * 128 * bpc).values())[:4]
+    assert path(4096, 4096, 8, 28672, 2, 2) == ("moe_tokn_kernel<up>", "moe_tokn_kernel<down>", 3, False)
+    assert path(65536, 4096, 128, 3072, 8, 1) == ("moe_up_dual_bf16_kernel", "moe_tokn_kernel<down>", 3, False)
+    assert path(32768, 2048, 128, 4096, 4, 1) == ("moe_tokn_kernel<up>", "moe_tokn_kernel<down>", 4, False)     # 128 MB of x
+    assert path(6000, 2048, 128, 768, 8, 1) == ("moe_up_bf16_kernel", "moe_down_bf16_kernel", 2, False)
+    assert path(2000, 2048, 128, 768, 8, 1) == ("moe_up_bf16_kernel", "moe_down_bf16_kernel", 3, False)
+    monkeypatch.setenv("PMOE_TOKN", "0")
+    assert path(4096, 4096, 8, 28672, 2, 2) == ("moe_pair_bf16_kernel<up>", "moe_pair_bf16_kernel<down>", 6, True)
