@@ -86,16 +86,17 @@ def spread(T, n):
 
 
 def test_c1_mixtral_cta_pairs_full_size(monkeypatch):
-    """Configuration 1 exactly as the benchmark runs it: bpc=2 (CTA pairs), stages=4, with the half-empty last
-    pairs as single blocks on the one-CTA kernels (default) and as pairs."""
+    """Configuration 1 exactly as the benchmark runs it (bpc=2, stages=4: token-N kernels), and on the row-M CTA pairs, with
+    the half-empty last pairs as single blocks on the one-CTA kernels and as pairs (setting PMOE_PAIR_TAILS selects them)."""
     T, K, E, N, k = 4096, 4096, 8, 28672, 2
     x, w1, w2, ids, wts = device_case(T, K, E, N, k, seed=7)
     toks = spread(T, 16)
     ref = oracle_rows(toks, x, w1, w2, ids, wts)
     one = run_bf16(x, w1, w2, ids, wts, bpc=1)
     assert O.max_rel_to_peak(one[toks].cpu(), ref) <= TOL
-    for tails in ("1", "0"):
-        monkeypatch.setenv("PMOE_PAIR_TAILS", tails)
+    for tails in (None, "1", "0"):
+        if tails is not None:
+            monkeypatch.setenv("PMOE_PAIR_TAILS", tails)
         out = run_bf16(x, w1, w2, ids, wts, bpc=2)
         assert torch.isfinite(out.float()).all()
         assert O.max_rel_to_peak(out.cpu(), one.cpu().float()) <= TOL
