@@ -1598,7 +1598,9 @@ Decisions decide(const Problem &p) {
     // saves the row-gathered copy in HBM, whose power counts on a chip at its cap: it stays where the rows are long beside
     // the layer's width (row-M / token-N: K = 4096, N = 3072, 524288 Zipf rows 18.8 / 20.0 ms at the cap, though 18.1 /
     // 16.7 ms on a cool chip; K = 2688, N = 1280 1916 / 2010 us; but K = 2304, N = 2816 4294 / 3878 us; K = 5248, N = 5120
-    // 2428 / 1961; K = 2176, N = 2048 319 / 282).
+    // 2428 / 1961; K = 2176, N = 2048 319 / 282). The first of these, tens of ms of calls at the cap, draws the line: 143
+    // random layers with 8 K > 9 N timed over 40 ms back to back were on the token-N kernels alone 0.84 (K < 1.4 N), 0.86
+    // (< 2 N), 0.92 (< 3 N) and 0.98 of the row-M time, with the token-N down kernel only 0.96, 0.97, 0.99 and 1.00.
     // Where the row-M gate/up tiles of up to 1024 rows per expert fill one round of the SMs, each with as many MMAs as a
     // tile of a CTA pair, the row copy and the planning are all that the token-N kernels add, unless K is long (row-M /
     // token-N, us: 5 experts, 958 rows each, K = 1536, N = 768 38 / 48; 4, 800, K = 1408, N = 512 34 / 42; 6, 477, K = 2304,
