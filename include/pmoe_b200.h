@@ -97,8 +97,10 @@ size_t pmoe_moe_align_static_capacity_bytes(void);
  *
  *   x   bf16[M, K]        w   bf16[E, N, K]  (rows [0,N/2) gate, [N/2,N) up)     w2  bf16[E, K, N/2]
  *   out bf16[M, K]        sorted_token_ids int32[sorted_num], expert_ids int32[>= sorted_num/128],
- *   num_tokens_post_padded int32[1], topk_weights fp32[M*top_k] (indexed by pair id)
- *   block_m == 128; (block_n, warp_n) in {(32,8), (64,4)}; stages 1..5 (<= 4 when split);
+ *   num_tokens_post_padded int32[1], topk_weights fp32[M*top_k] (indexed by pair id). A table may list a pair in
+ *   several rows: every row contributes.
+ *   block_m == 128; (block_n, warp_n) in {(32,8), (64,4)}; stages 1..5 (<= 4 when split): checked always, used where
+ *   pmoe_debug_bf16_route names no token-N kernel;
  *   bpc in {1, 2} (2 = two-CTA MMA; needs moe_align run with the same bpc); cpc == 1;
  *   K % 128 == 0, N % 256 == 0.
  *   split == 0: one GEMM launch (gate/up + down per tile, split-K partials reduced in an fp32 workspace
@@ -188,7 +190,7 @@ enum { PMOE_DTYPE_F32 = 0, PMOE_DTYPE_BF16 = 1 };
 int pmoe_route_topk(const void *logits, int logits_dtype, int T, int num_experts, int top_k, int renormalize,
                     int32_t *topk_ids, float *topk_weights, pmoe_stream_t stream);
 /* Router and moe_align in one call: as pmoe_route_topk followed by pmoe_moe_align_ws on its topk_ids (same outputs,
- * bit for bit); a decode batch (T <= 32) is routed and aligned by one launch.
+ * bit for bit); a decode batch (T <= 32, or 8 with more than 256 experts) is routed and aligned by one launch.
  * workspace: pmoe_moe_align_workspace_bytes(T * top_k, num_experts) bytes. Up to 4096 ids (16384 with at most 256
  * experts) may come without: one CTA then aligns them, more slowly. */
 int pmoe_route_topk_align(const void *logits, int logits_dtype, int T, int num_experts, int top_k, int renormalize,

@@ -95,8 +95,7 @@ def route_topk(logits, top_k, renormalize=True):
 
 def route_topk_align(logits, top_k, renormalize=True, block_m=128, bpc=1):
     """``route_topk`` and ``moe_align`` in one call: ``(topk_ids, topk_weights, sorted_token_ids, expert_ids,
-    num_tokens_post_padded)``. Above the single-CTA sizes one kernel routes the tokens and counts its own ids per
-    expert, so the histogram pass of ``moe_align`` and one launch disappear."""
+    num_tokens_post_padded)``. A decode batch (up to 32 tokens, 8 with more than 256 experts) takes one launch."""
     return torch.ops.prime_moe.route_topk_align(logits, top_k, renormalize, block_m, bpc)
 
 

@@ -82,14 +82,14 @@ int l2_prefetch_distance();
 
 // PMOE_SHORT_A=0 switches off the short TMA boxes (row blocks with few routed rows move only those rows of the
 // A operand and of the activation tile); read on every call so that tests can compare both settings
-int short_boxes_mode();
+int short_boxes_mode();   // bit 0: loads, bit 1: activation stores
 
 // bpc = 2 runs the half-empty last pair of an expert as a single block on the one-CTA kernels (PMOE_PAIR_TAILS=0:
 // as a pair, like every other one)
 bool pair_tails_enabled();
 
 // PMOE_DUAL=0/1 forces one / two row blocks per tile in the one-CTA bf16 gate/up kernel; unset = -1 = by size
-int dual_blocks_mode();   // bit 0: loads, bit 1: activation stores
+int dual_blocks_mode();
 
 // The bf16 split pipeline runs on the token-N kernels (moe_bf16_tokn.cu) where they are the faster ones, but not with
 // PMOE_TOKN=0, nor when one of the switches of the row-M kernels above is set (a caller who sets one means those
