@@ -366,6 +366,8 @@ int pmoe_debug_bf16_route(int M, int K, int N, int num_experts, int top_k, int b
 /* ... and the backward pass: 1 = weight gradients on CTA pairs, 2 = the row-space GEMMs as well, or their sum; 4 = the
  * row-space GEMMs on the token-N kernels. */
 int pmoe_debug_backward_route(int T, int K, int N, int num_experts, int top_k);
+/* ... and the token-N bf16 down kernel: 1 = it adds its rows by bulk reductions, 0 = by vector reductions. */
+int pmoe_debug_tokn_bulk_down(int M, int N, int num_experts, int top_k);
 
 #ifdef __cplusplus
 }

@@ -13,17 +13,17 @@
 //               16-lane TMEM loads give a thread both. SwiGLU -> bf16 -> staging -> TMA store.
 //   down        tile = item x 256 output columns, 128 per CTA; accumulator * routing weight -> bf16 -> transposed through the
 //               warp's own staging buffer -> 16-byte vector reductions into out[token] by the epilogue warps themselves.
-//               (A store warp's 256-byte bulk reductions, one a routed row, cost 31 ns each and SM and needed 51 KB of
-//               staging: 8 experts, 128 rows each, K = 4096, N = 512 29.6 -> 25.0 us; equal from H = 768 on in bf16, where
-//               the MMAs cover either; mxfp8, T = 5003, K = 2048, N = 1536, top_k = 8 133 -> 101 us.)
+//               (A store warp's 256-byte bulk reductions, one a routed row, cost 31 ns each and SM and need 51 KB of staging:
+//               8 experts, 128 rows each, K = 4096, N = 512 29.6 -> 25.0 us; mxfp8, T = 5003, K = 2048, N = 1536, top_k = 8
+//               133 -> 101 us. Long rows take them all the same: tokn_bulk_down().)
 //
 //   backward    row-space GEMMs where an expert has few rows: tile = row block x 256 output columns, the rows by TMA from the
 //               sorted copies, results rows of 16-byte stores through the warp's own tiles (D_ACT: SwiGLU derivative there).
 //
 // Warp roles: warp 0 TMA producer, warp 1 TMEM owner + MMA issuer (even CTA), warps 2-9 epilogue in two groups of four
-// (a group takes every second 32-row chunk of the accumulator), gate/up: warps 10-11 one store warp per group: it waits for
-// a staged chunk, issues the bulk stores (mxfp8: quantises it) and hands the buffer back, so that the epilogue warps never
-// wait for a store to be read; four warps copy the routed rows of x straight into the ring (cp.async; no row-sorted copy of x
+// (a group takes every second 32-row chunk of the accumulator), gate/up and bulk reductions: warps 10-11 one store warp per
+// group: it waits for a staged chunk, issues the bulk stores (mxfp8: quantises it) and hands the buffer back, so that the
+// epilogue warps never wait for a store to be read; gate/up: four warps copy the routed rows of x straight into the ring (cp.async; no row-sorted copy of x
 // in HBM, which cost 75 of 645 us at T = 8192, K = 2048, N = 1536, top_k = 8) and one publishes what has landed. Two
 // accumulators in TMEM; every wait is bounded (ptx.cuh).
 //
@@ -50,14 +50,15 @@ __device__ int g_status_tokn = 0;
 namespace {
 
 constexpr int BM = kBlockM;
-// What a launch contracts. The first two are the forward pass, the others the row-space GEMMs of the backward pass. D_ACT
+// What a launch contracts. The first three are the forward pass, the others the row-space GEMMs of the backward pass. D_ACT
 // and D_XS read their weights with the output dimension contiguous (M-major operand: two 64 x 64 boxes a CTA and k-step).
 enum : int {
     UP = 0,       // gate | up of the routed rows, SwiGLU
-    DOWN = 1,     // act . W2[e]^T, weighted, added into out[token]
-    GATE_UP = 2,  // rows of x . W1[e]^T -> rows of the pre-activations
-    D_ACT = 3,    // rows of d_out . W2[e], SwiGLU derivative -> d_gate | d_up, weight * act, d_weight
-    D_XS = 4,     // d_gate | d_up . W1[e] -> rows of d_xs
+    DOWN = 1,     // act . W2[e]^T, weighted, added into out[token] by vector reductions ...
+    DOWN_BULK = 2,   // ... by bulk reductions
+    GATE_UP = 3,  // rows of x . W1[e]^T -> rows of the pre-activations
+    D_ACT = 4,    // rows of d_out . W2[e], SwiGLU derivative -> d_gate | d_up, weight * act, d_weight
+    D_XS = 5,     // d_gate | d_up . W1[e] -> rows of d_xs
 };
 constexpr uint32_t A_BYTES = 128 * 128;          // 16 KB: 128 weight rows x 128 bytes of K per CTA and k-step
 template <bool kMx> constexpr int BK = kMx ? 128 : 64;            // K elements of a k-step (128 bytes)
@@ -70,13 +71,16 @@ constexpr int SCALE_WARP = STORE_WARP + 2;       // ... mxfp8: a scale warp and 
 template <bool kMx> constexpr int GATHER_WARP = SCALE_WARP + (kMx ? 2 : 0);   // ... four for the rows of x and their publisher
 constexpr int GATHER_THREADS = 128;
 template <int kMode, bool kMx>
-constexpr int THREADS = (kMode != UP ? STORE_WARP : GATHER_WARP<kMx> + GATHER_THREADS / 32 + 1) * 32;
+constexpr int THREADS = (kMode == UP ? GATHER_WARP<kMx> + GATHER_THREADS / 32 + 1 : STORE_WARP + (kMode == DOWN_BULK ? 2 : 0)) * 32;
 constexpr int CHUNK = 32;                        // rows per staged chunk
 constexpr int UP_BUFS = 4;        // staging buffers per epilogue group
 constexpr uint32_t UP_BUF_BYTES = CHUNK * 128;           // 32 rows x 64 activation columns, 128-byte swizzle
 // down: a warp's own 32 routed rows x 32 output columns, a row padded so that neither stmatrix nor 16-byte loads conflict
 constexpr uint32_t DOWN_ROW_BYTES = 64 + 16;
 constexpr uint32_t DOWN_BUF_BYTES = CHUNK * DOWN_ROW_BYTES;
+constexpr int BULK_BUFS = 3;                                      // ... bulk reductions: a group's 32 rows x 128 columns
+constexpr uint32_t BULK_ROW_BYTES = 256 + 16;
+constexpr uint32_t BULK_BUF_BYTES = CHUNK * BULK_ROW_BYTES;
 constexpr int KEEP_BUFS = 2;                                      // gate/up with kept pre-activations: activation, gate
 constexpr uint32_t KEEP_BUF_BYTES = 3 * UP_BUF_BYTES;             // and up chunks in one buffer
 // mxfp8 gate/up: the staged chunk is the fp32 SwiGLU value, quantised by the store warps; 64 activations a row, padded so
@@ -91,9 +95,10 @@ constexpr int SFA_BATCHES = 8;                   // gate/up: a ring of its own f
 constexpr uint32_t SFA_BYTES = SFA_BATCHES * 2 * SF_TILE;
 constexpr uint32_t SF_TMEM = 384;                // TMEM columns of the scales: eight regions of 4 (weights) + 8 (rows)
 template <int kMode, bool kKeep, bool kMx>
-constexpr int BUFS = kMode != UP ? EPI_WARPS / 2 : kMx ? MX_UP_BUFS : kKeep ? KEEP_BUFS : UP_BUFS;
+constexpr int BUFS = kMode == DOWN_BULK ? BULK_BUFS : kMode != UP ? EPI_WARPS / 2 : kMx ? MX_UP_BUFS : kKeep ? KEEP_BUFS : UP_BUFS;
 template <int kMode, bool kKeep, bool kMx>
-constexpr uint32_t BUF_BYTES = kMode == D_ACT ? 5 * D_ACT_TILE : kMode != UP ? DOWN_BUF_BYTES : kMx ? MX_UP_BUF_BYTES : kKeep ? KEEP_BUF_BYTES : UP_BUF_BYTES;
+constexpr uint32_t BUF_BYTES = kMode == D_ACT ? 5 * D_ACT_TILE : kMode == DOWN_BULK ? BULK_BUF_BYTES : kMode != UP ? DOWN_BUF_BYTES
+                               : kMx ? MX_UP_BUF_BYTES : kKeep ? KEEP_BUF_BYTES : UP_BUF_BYTES;
 constexpr uint32_t BAR_BYTES = 768;
 constexpr uint32_t SMEM_LIMIT = 232448;
 constexpr int ST_BAD_PAIR = 8;                   // bpc = 2 table whose 256-row pair holds two experts
@@ -438,7 +443,8 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const __grid_constant__ CUtensorMap map_rows16, const __grid_constant__ CUtensorMap map_act,
                 const __grid_constant__ CUtensorMap map_gu, const Args a) {
     extern __shared__ uint8_t smem_raw[];
-    constexpr bool kUp = kMode == UP, kBackward = kMode >= GATE_UP, kMMajor = kMode >= D_ACT;
+    constexpr bool kUp = kMode == UP, kBulk = kMode == DOWN_BULK, kDown = kMode == DOWN || kBulk, kBackward = kMode >= GATE_UP;
+    constexpr bool kMMajor = kMode >= D_ACT;
     constexpr int kBufs = BUFS<kMode, kKeep, kMx>;
     constexpr uint32_t kBufBytes = BUF_BYTES<kMode, kKeep, kMx>;
     constexpr int kBK = BK<kMx>;
@@ -547,10 +553,10 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                                          ((w.expert * a.K + w.n_tile * 256) / 128 + static_cast<int>(rank)) * ksteps + ks);
                 };
                 // down: the weights of the first round of slots do not depend on gate/up, only their rows do
-                const int early = kMode == DOWN && t == first ? min(a.stages, ksteps) : 0;
+                const int early = kDown && t == first ? min(a.stages, ksteps) : 0;
                 for (int ks = 0; ks < early; ++ks) load_weights(ks, ks);
                 const long long before = issued;
-                if (kMode == DOWN && t == first && a.use_pdl) pdl_wait_primary();
+                if (kDown && t == first && a.use_pdl) pdl_wait_primary();
                 for (int ks = 0; ks < ksteps; ++ks) {
                     ok = mbar_wait(sm.empty(s), ph ^ 1, status, ST_TIMEOUT_EMPTY);
                     if (!ok) break;
@@ -658,6 +664,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // (One column a thread and 2-byte stores with a shuffle per element was bound by them: 4 us a tile.)
         const uint32_t mat = lane >> 3, mrow = lane & 7;
         const uint32_t off = kMode == D_ACT ? tile64(mrow, mat)
+                             : kBulk ? mrow * BULK_ROW_BYTES + (quarter * 32 + 8 * mat) * 2
                              : !kUp ? mrow * DOWN_ROW_BYTES + 16 * mat
                              : kMx ? 2 * (lane & 3) * MX_UP_ROW_BYTES + (quarter * 16 + (lane >> 2)) * 4
                                    : (8 * (mat >> 1) + mrow) * 128 + (((2 * quarter + (mat & 1)) ^ mrow) << 4);
@@ -680,7 +687,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             }
             return true;
         };
-        if (kMode == DOWN) fetch_rows(a.row_info, next, grp, lane, info_next);
+        if (kDown) fetch_rows(a.row_info, next, grp, lane, info_next);
         if (kMode == D_ACT) fetch_pairs(a, next, grp, lane, info_next);
         if (kMode == DOWN && a.use_pdl) pdl_wait_primary();      // gate/up zeroes `out`
         for (int t = first; t < num_tiles && ok; t += step, ++it_n) {
@@ -688,7 +695,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             next = fetch(t + step);
             const int chunks = w.rows / CHUNK;
             const int buf = it_n & 1;
-            if (kMode == DOWN || kMode == D_ACT) {
+            if (kDown || kMode == D_ACT) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) info[j] = info_next[j];
             }
@@ -700,7 +707,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = tmem_base + buf * ACC_COLS<kMx>;
-            if (kMode == DOWN) fetch_rows(a.row_info, next, grp, lane, info_next);
+            if (kDown) fetch_rows(a.row_info, next, grp, lane, info_next);
             if (kMode == D_ACT) fetch_pairs(a, next, grp, lane, info_next);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -791,7 +798,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                     continue;
                 }
-                if (!kUp) {
+                if (kMode == DOWN) {
                     const uint32_t mine = sm.staging + (warp - 2) * DOWN_BUF_BYTES;
                     tmem_ld_wait();
                     __syncwarp();                   // the previous chunk has been read
@@ -850,6 +857,17 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         stmatrix_x4_trans(base + p * 16 * 128, pack_bf16x2(lo[8 * p], lo[8 * p + 1]),
                                           pack_bf16x2(lo[8 * p + 2], lo[8 * p + 3]), pack_bf16x2(lo[8 * p + 4], lo[8 * p + 5]),
                                           pack_bf16x2(lo[8 * p + 6], lo[8 * p + 7]));
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {   // 8 routed rows x 32 output columns
+                        const int r = 8 * q + 2 * (lane & 3);
+                        const float w0 = __int_as_float(__shfl_sync(0xffffffffu, info[j].y, r));
+                        const float w1 = __int_as_float(__shfl_sync(0xffffffffu, info[j].y, r + 1));
+                        stmatrix_x4_trans(base + q * 8 * BULK_ROW_BYTES, pack_bf16x2(w0 * lo[4 * q], w1 * lo[4 * q + 1]),
+                                          pack_bf16x2(w0 * lo[4 * q + 2], w1 * lo[4 * q + 3]),
+                                          pack_bf16x2(w0 * hi[4 * q], w1 * hi[4 * q + 1]),
+                                          pack_bf16x2(w0 * hi[4 * q + 2], w1 * hi[4 * q + 3]));
+                    }
                 }
                 if (!kMx) fence_proxy_async_smem();
                 __syncwarp();
@@ -985,17 +1003,25 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
         }
         __syncwarp();
-    } else if (kUp) {
+    } else if (kUp || kBulk) {
         // ---------------- store warps ----------------
         const int grp = warp - STORE_WARP;
         uint32_t chunk_n = 0;
         bool ok = true;
         Tile w, next = fetch(first);
+        int2 info[4], info_next[4];
+        if (kBulk) fetch_rows(a.row_info, next, grp, lane, info_next);
+        if (kBulk && a.use_pdl) pdl_wait_primary();      // gate/up zeroes `out`
         for (int t = first; t < num_tiles && ok; t += step) {
             w = next;
             next = fetch(t + step);
             const int chunks = w.rows / CHUNK;
-            const int col0 = w.n_tile * 128 + static_cast<int>(rank) * 64;
+            const int col0 = kBulk ? w.n_tile * 256 + static_cast<int>(rank) * 128 : w.n_tile * 128 + static_cast<int>(rank) * 64;
+            if (kBulk) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) info[j] = info_next[j];
+                fetch_rows(a.row_info, next, grp, lane, info_next);
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int ch = grp + 2 * j;
@@ -1035,7 +1061,10 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     ++chunk_n;
                     continue;
                 }
-                if (lane == 0) {
+                if (kBulk) {
+                    if (info[j].x >= 0 && col0 < a.K)
+                        bulk_reduce_add_bf16(a.out + static_cast<size_t>(info[j].x) * a.K + col0, base + lane * BULK_ROW_BYTES, 256);
+                } else if (lane == 0) {
                     tma_store_2d(&map_act, base, col0, w.row0 + ch * CHUNK);
                     if (kKeep) {
                         tma_store_2d(&map_gu, base + UP_BUF_BYTES, col0, w.row0 + ch * CHUNK);
@@ -1125,6 +1154,17 @@ static int tokn_cap(const ToknProblem &p) {
     // 416; K = 3584, N = 10240, 106 rows 301 / 270; below 32 rows 64 and 192 differ by 3 % either way)
     if (p.w_scales) return rows <= 32ll * p.E ? 64 : 192;
     return rows <= 32ll * p.E ? 64 : rows <= 112ll * p.E ? 128 : 256;
+}
+
+// How the down kernel adds its rows. Bulk reductions move 256 bytes an operation instead of 16, which counts at the power
+// cap: with many rows and a contraction long enough to cover their 31 ns each (whole call, vector / bulk, us, runs of 1 s back
+// to back: K = 4096, N = 3072, 524288 Zipf rows 18202 / 17875, 32 experts, 4096 rows each 4196 / 4163; K = 5120, N = 2048, 2200
+// rows each 1018 / 1001; K = 6144, N = 5120, 2048 rows each 12118 / 11928). Shorter contractions do not cover them (N = 1536,
+// 512 rows 677 / 682, 11000 rows 1.02; N = 1280, 3277 rows 1293 / 1352; N = 768, 4096 rows 1294 / 1441); at 512 rows per expert
+// the two are within 1 % of each other, and below the staging's 51 KB, taken from the ring, cost more (1.00 - 1.09).
+// mxfp8's MMAs take half the time: vector reductions everywhere (K = 2048, N = 1536, 5003 tokens 101 / 133).
+static bool tokn_bulk_down(int M, int N, int E, int top_k) {
+    return N >= 2048 && static_cast<long long>(M) * top_k >= 1024ll * E;
 }
 
 // the count, at most two pieces per 128-row block (cap 64) and the row info
@@ -1227,7 +1267,8 @@ int run_tokn(const ToknProblem &p, void *act, void *items, int phases, cudaStrea
                 return rc;
             rc = launch<DOWN, false, true>(w2, actb, act16, sfa, sfw, dn, cap, tiles, stream);
         } else {
-            rc = launch<DOWN>(w2, actb, act16, act_st, act_st, dn, cap, tiles, stream);
+            rc = tokn_bulk_down(p.M, p.N, p.E, p.top_k) ? launch<DOWN_BULK>(w2, actb, act16, act_st, act_st, dn, cap, tiles, stream)
+                              : launch<DOWN>(w2, actb, act16, act_st, act_st, dn, cap, tiles, stream);
         }
         if (rc) return rc;
     }
@@ -1293,3 +1334,7 @@ int status_fetch_tokn(int *value, bool reset) {
 }
 
 }  // namespace pmoe
+
+extern "C" int pmoe_debug_tokn_bulk_down(int M, int N, int num_experts, int top_k) {
+    return pmoe::tokn_bulk_down(M, N, num_experts, top_k) ? 1 : 0;
+}

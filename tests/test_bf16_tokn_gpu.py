@@ -74,6 +74,16 @@ def test_matrix_sizes_at_tile_edges(K, N):
     run((40, 0, 130, 7), K, N, 1)
 
 
+# down kernel with bulk reductions (N >= 2048, 1024 rows per expert on average): pieces of 32 to 256 rows, K % 256 == 128,
+# more k-steps than ring slots, chunks of one and of both epilogue groups
+@pytest.mark.parametrize("counts,K,N", [((1024,), 128, 2048), ((3000, 0, 72), 384, 2304), ((1, 4095, 33, 0), 256, 2048),
+                                        ((1900, 161, 1300, 735), 1152, 2048)])
+def test_down_kernel_with_bulk_reductions(counts, K, N):
+    from prime_flash_moe_b200 import capi
+    assert capi.lib().pmoe_debug_tokn_bulk_down(sum(counts), N, len(counts), 1) == 1
+    run(counts, K, N, 1)
+
+
 def test_an_expert_seen_in_separate_runs_and_holes_inside_a_block():
     """A hand-made routing table: expert 0 in two separate runs, and a block whose rows are not contiguous."""
     from prime_flash_moe_b200 import capi
