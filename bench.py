@@ -357,8 +357,8 @@ def bf16_path(lib, T, K, N, E, k, bpc, sorted_num):
     reports them: names of the gate/up and down kernels, launches per call, whether half-empty row-block pairs run in
     launches of their own, and what runs under every phase mask beside the kernel it names (timed with it)."""
     route = lib.pmoe_debug_bf16_route(T, K, N, E, k, bpc, 0)
-    token_n, two_block, pairs = route & 1, route & 4, route & 8
-    if token_n:
+    token_n_up, token_n_down, two_block, pairs = route & 1, route & 2, route & 4, route & 8
+    if token_n_up:
         return {"up": "moe_tokn_kernel<up>", "down": "moe_tokn_kernel<down>", "launches": 3, "tails": False,
                 "includes": "plan_kernel (up, down)"}
     if pairs:
@@ -369,7 +369,9 @@ def bf16_path(lib, T, K, N, E, k, bpc, sorted_num):
     if os.environ.get("PMOE_PREGATHER") == "0":
         pre_pass = False
     return {"up": "moe_up_dual_bf16_kernel" if two_block else "moe_up_bf16_kernel",
-            "down": "moe_down_bf16_kernel", "launches": 2 + int(pre_pass), "tails": False, "includes": None}
+            "down": "moe_tokn_kernel<down>" if token_n_down else "moe_down_bf16_kernel",
+            "launches": 2 + int(pre_pass) + (1 if token_n_down else 0), "tails": False,
+            "includes": "plan_kernel (down)" if token_n_down else None}
 
 
 def mx_up_kernel():

@@ -187,6 +187,11 @@ bool token_n_enabled() {   // read on every call, in one pass over the environme
     return !row_m;
 }
 
+bool token_n_forced() {
+    const char *e = getenv("PMOE_TOKN");
+    return e && e[0] == '1';
+}
+
 static int g_phase_mask = 7;
 int phase_mask() { return g_phase_mask; }
 

@@ -92,8 +92,10 @@ bool pair_tails_enabled();
 int dual_blocks_mode();
 
 // The bf16 split pipeline runs on the token-N kernels (moe_tokn.cu), but not with PMOE_TOKN=0, nor when one of the
-// switches of the row-M kernels above is set (a caller who sets one means those kernels) without PMOE_TOKN=1
+// switches of the row-M kernels above is set (a caller who sets one means those kernels); PMOE_TOKN=1 takes them at every
+// size and whatever the switches
 bool token_n_enabled();
+bool token_n_forced();
 
 // which launches of a split pipeline run (pmoe_debug_set_phase_mask): 1 gather, 2 gate/up, 4 down; 8 = without the
 // single-block tail launches of the bpc = 2 pipeline (to time the CTA-pair kernels alone)

@@ -1568,22 +1568,30 @@ struct Decisions {
     bool tails;       // bpc == 2: pair / tail lists written and read
     bool token_n;     // the token-N kernels run instead (work items written and read)
     bool dual;        // bpc == 1, not token_n: two row blocks per gate/up tile (shared weight slots)
+    bool token_n_down;   // ... and the token-N down kernel after it (work items written and read)
 };
 Decisions decide(const Problem &p) {
     Decisions d{};
-    // Token-N kernels, whatever the size: since their gate/up kernel gathers the rows of x itself they are the faster ones
-    // nearly everywhere. Whole call against the row-M kernels: 0.70 - 1.00 on 80 random layers (K 1024 - 7168, N 512 - 19968,
-    // 9 - 235 experts, 1 - 64586 tokens; us: K = 1024, N = 1792, 29800 rows per expert 2432 / 1702; K = 1408, N = 512, 169
-    // rows 81 / 60; K = 4096, N = 3072, 524288 Zipf rows 19294 / 17657), one at 1.06. Where the gate/up tiles are 1.0 to 1.4
-    // times the CTA pairs (one round of the SMs, two of the pairs) they still win on 50 of 60 layers (0.65 - 0.99; K = 4096,
-    // N = 8192, 4 experts, 16 tokens 104 / 76) and lose 5 - 8 % on the others (K = 4864, N = 4096, 5 experts, 40 rows each
-    // 1.07), which no size tells apart. With live_rows (M is the capacity of a buffer, the planner sees the rows in use)
-    // 0.60 - 0.90 (capacity 32768, K = 4096, N = 3072, 16 experts: 256 rows in use 206 / 130, 8192 460 / 352), but one
-    // expert, N = 28672, 32 rows in use 137 / 172.
+    // Token-N kernels, nearly whatever the size, since their gate/up kernel gathers the rows of x itself. Whole call against the
+    // row-M kernels: 0.70 - 1.00 on 110 random layers (K 1024 - 7168, N 512 - 26112, 1 - 253 experts, 1 - 33129 tokens; us:
+    // K = 2304, N = 768, 9 experts, 305 rows each 41 / 31; K = 4096, N = 3072, 32 experts, 4096 rows each 4388 / 4163), four at
+    // 1.02 - 1.07. Where the gate/up tiles are 1.0 to 2.0 times the CTA pairs (one round of the SMs, two of the pairs) they
+    // still win on 34 of 38 layers (0.77 - 0.99) and lose 1 - 8 % on the others (K = 3200, N = 3328, 6 rows on 6 experts 52 /
+    // 56), which no size tells apart.
+    // The largest calls stay with the two-block gate/up kernel, which gathers the rows as well, followed by the token-N down
+    // kernel: these hold the power cap longest, and are the faster ones there (token-N / these, ms, runs of half a second back
+    // to back: K = 4096, N = 3072, 128 experts, 524288 rows, even 18.56 / 17.67, Zipf 17.87 / 17.65, on a hotter chip 19.52 /
+    // 18.43 and 19.17 / 18.71; with 32 experts 16.48 / 16.83). At 3.8e12 to 4.4e12 rows * K * N the two are level (0.96 - 1.03
+    // on six layers, one of them 1.02 on one chip and 0.98 on another), below that token-N is the faster one: 0.90 - 0.98 on
+    // 14 layers (K = 4096, N = 3072, 128 experts, 262144 rows 9.13 / 9.54; K = 6144, N = 5120, 64 experts, 65536 rows 6.08 /
+    // 6.82). On layers with 8 K <= 9 N and as CTA pairs (bpc = 2) it is level with or faster than the row-M kernels at every
+    // size (0.94 - 1.01 on eleven). With live_rows M is a capacity, which says nothing about the rows in use.
     // Results addressed through out_rows may live in a peer's memory: they stay with the row-M kernels.
-    d.token_n = token_n_enabled() && !call_extras().out_rows;
-    if (d.token_n) return d;
     const long long rows = static_cast<long long>(p.M) * p.top_k;
+    const bool long_rows = p.bpc == 1 && p.N >= 2048 && 8ll * p.K > 9ll * p.N && rows >= 1024ll * p.E &&
+                           rows * p.K >= 4500000000000ll / p.N && !call_extras().live_rows;
+    d.token_n = token_n_enabled() && !call_extras().out_rows && (token_n_forced() || !long_rows);
+    if (d.token_n) return d;
     d.a_mode = a_operand_mode();
     // auto: the in-kernel LSU gather pays off when the row-gather pre-pass is a visible share of the step (its
     // cost is ~250/N of a compute-bound step) and the step is compute-bound (>= 256 routed rows per expert on
@@ -1599,6 +1607,7 @@ Decisions decide(const Problem &p) {
     // rows per expert, where more pairs straddle two experts)
     const int dual_env = dual_blocks_mode();
     d.dual = p.bpc == 1 && d.a_mode != 0 && (dual_env < 0 ? rows >= 1024ll * p.E : dual_env != 0);
+    d.token_n_down = long_rows && d.dual && token_n_enabled() && !call_extras().out_rows;
     return d;
 }
 
@@ -1845,6 +1854,8 @@ int run(const Problem &p, void *workspace, size_t workspace_bytes, cudaStream_t 
         }
         return PMOE_OK;
     }
+    const ToknProblem tdown{p.x, p.w, p.w2, p.out, p.sorted_ids, p.expert_ids, p.npp, p.topk_weights, extras.live_rows,
+                            nullptr, p.top_k, p.M, p.K, p.N, p.E, p.sorted_num, p.bpc};
     if ((phases & 2) && dec.dual) {
         Args up = a;
         up.zero_out = extras.out_rows ? 0 : 1;
@@ -1892,6 +1903,7 @@ int run(const Problem &p, void *workspace, size_t workspace_bytes, cudaStream_t 
         cfg.numAttrs = up.use_pdl ? 1 : 0;
         PMOE_CUDA_OK(cudaLaunchKernelEx(&cfg, up_kernel, map_x, map_w1, map_act, map_x_short, map_act_short, up));
     }
+    if ((phases & 4) && dec.token_n_down) return run_tokn(tdown, workspace, ws_base + lay.items, 4, stream);
     if (phases & 4) {
         Args dn = a;
         dn.use_pdl = (pdl_enabled() && (phases & 2)) ? 1 : 0;
@@ -1951,7 +1963,7 @@ extern "C" size_t pmoe_debug_bf16_workspace_extent(int M, int K, int N, int num_
     size_t end = rows * (N / 2) * 2;                                  // activation
     if (d.pregather) end = std::max(end, lay.x_sorted + rows * K * 2);
     if (d.tails) end = std::max(end, lay.lists + (2 * (rows / 256) + 2) * sizeof(int32_t));
-    if (d.token_n) end = std::max(end, lay.items + tokn_items_bytes(sorted_num));
+    if (d.token_n || d.token_n_down) end = std::max(end, lay.items + tokn_items_bytes(sorted_num));
     return end;
 }
 
@@ -1964,7 +1976,7 @@ extern "C" int pmoe_debug_bf16_route(int M, int K, int N, int num_experts, int t
     const Decisions d = decide(p);
     call_extras() = CallExtras{};
     return (d.token_n ? PMOE_ROUTE_TOKEN_N_UP | PMOE_ROUTE_TOKEN_N_DOWN : 0) | (d.dual ? PMOE_ROUTE_TWO_BLOCK_UP : 0) |
-           (bpc == 2 && !d.token_n ? PMOE_ROUTE_CTA_PAIRS : 0);
+           (d.token_n_down ? PMOE_ROUTE_TOKEN_N_DOWN : 0) | (bpc == 2 && !d.token_n ? PMOE_ROUTE_CTA_PAIRS : 0);
 }
 
 extern "C" int pmoe_fused_moe_bf16_ws(const void *x, const void *w, const void *w2, void *out,
