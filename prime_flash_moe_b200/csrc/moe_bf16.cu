@@ -1585,12 +1585,21 @@ Decisions decide(const Problem &p) {
     // on six layers, one of them 1.02 on one chip and 0.98 on another), below that token-N is the faster one: 0.90 - 0.98 on
     // 14 layers (K = 4096, N = 3072, 128 experts, 262144 rows 9.13 / 9.54; K = 6144, N = 5120, 64 experts, 65536 rows 6.08 /
     // 6.82). On layers with 8 K <= 9 N and as CTA pairs (bpc = 2) it is level with or faster than the row-M kernels at every
-    // size (0.94 - 1.01 on eleven). With live_rows M is a capacity, which says nothing about the rows in use.
+    // size (0.94 - 1.01 on eleven).
+    // With live_rows M is a capacity, which says nothing about the rows in use. Token-N all the same (capacity 8192 or 16384,
+    // 64 - 512 rows in use 0.41 - 0.97 of the row-M time), but for one wide expert as CTA pairs: its down kernel has K / 256
+    // tiles whatever the rows, and its gate/up tiles take two rounds of the pairs where the single row block of a decode batch
+    // runs as one round of the SMs (K = 4096, N = 28672, capacity 32768, token-N / row-M, us: 32 rows 110 / 98, 128 rows 114 /
+    // 101; 200 rows 129 / 146, 2000 and more level; K = 7168, N = 20480, 32 rows 120 / 112; but N = 14336 62 / 73, and two
+    // experts of N = 14336 84 / 94).
     // Results addressed through out_rows may live in a peer's memory: they stay with the row-M kernels.
     const long long rows = static_cast<long long>(p.M) * p.top_k;
     const bool long_rows = p.bpc == 1 && p.N >= 2048 && 8ll * p.K > 9ll * p.N && rows >= 1024ll * p.E &&
                            rows * p.K >= 4500000000000ll / p.N && !call_extras().live_rows;
-    d.token_n = token_n_enabled() && !call_extras().out_rows && (token_n_forced() || !long_rows);
+    const int up_tiles = p.N / 256;
+    const bool one_wide_expert = call_extras().live_rows && p.E == 1 && p.bpc == 2 && p.K >= 3072 &&
+                                 2 * up_tiles > sm_count() && up_tiles <= sm_count();
+    d.token_n = token_n_enabled() && !call_extras().out_rows && (token_n_forced() || !(long_rows || one_wide_expert));
     if (d.token_n) return d;
     d.a_mode = a_operand_mode();
     // auto: the in-kernel LSU gather pays off when the row-gather pre-pass is a visible share of the step (its
