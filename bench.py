@@ -288,9 +288,10 @@ def roofline_mxfp8(args, capi, ops, tensors, ids, wts, out, cfg, peaks, whole_tf
     achieved = 2.0 * T * k * K * N / (per_kernel["moe_up_mxfp8"] * 1e-3) / 1e12
     peak, source = measure_mxfp8_peak(out.device)
     assert capi.device_status() == 0
-    return {"kernel": mx_up_kernel(), "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+    kernel = mx_up_kernel(lib, T, K, N, E, k, 1)
+    return {"kernel": kernel, "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "peak_source": source,
-            "traffic": 0.6565e9 if (args.config == "c2" and not args.tokens and mx_up_kernel() == "moe_up_mxfp8_kernel") else None,
+            "traffic": 0.6565e9 if (args.config == "c2" and not args.tokens and kernel == "moe_up_mxfp8_kernel") else None,
             "kernel_ms": per_kernel, "whole_op_frac": whole_tflops / peak}
 
 
@@ -374,11 +375,11 @@ def bf16_path(lib, T, K, N, E, k, bpc, sorted_num):
             "includes": "plan_kernel (down)" if token_n_down else None}
 
 
-def mx_up_kernel():
-    """The gate/up kernel the split mxfp8 operator takes under the current environment (timed together with plan_kernel)."""
-    other = ("PMOE_AGATHER", "PMOE_PREGATHER", "PMOE_DUAL", "PMOE_DOWN_BULK", "PMOE_PAIR_TAILS", "PMOE_SHORT_A")
-    row_m = os.environ["PMOE_TOKN"][:1] == "0" if "PMOE_TOKN" in os.environ else any(n in os.environ for n in other)
-    return "moe_up_mxfp8_kernel" if row_m else "moe_tokn_kernel<up, mxfp8>"
+def mx_up_kernel(lib, T, K, N, E, k, bpc):
+    """The gate/up kernel the split mxfp8 operator takes for a call of this size, as its launcher reports it (timed together
+    with plan_kernel, if that is the token-N one)."""
+    route = lib.pmoe_debug_mxfp8_route(T, K, N, E, k, bpc, 0)
+    return "moe_tokn_kernel<up, mxfp8>" if route & 1 else "moe_pair_mxfp8_kernel<up>" if route & 8 else "moe_up_mxfp8_kernel"
 
 
 def weight_streaming_roofline(roof, cfg, ids, per_kernel_up_ms, ms_step, peaks, mx, traffic):
@@ -546,7 +547,7 @@ def sweep_entry_ours(name, tokens, dtype, device, peaks, stages):
     assert capi.device_status() == 0, "a kernel recorded an error status"
     wb = (1.0 + 1.0 / 32) if mx else 2.0
     up_bytes = touched * N * K * wb + T * k * K * wb + T * k * (N // 2) * wb + T * K * 2
-    kernel = mx_up_kernel() if mx else path["up"]
+    kernel = mx_up_kernel(lib, T, K, N, E, k, bpc) if mx else path["up"]
     if T * k >= 256 * E:       # compute-bound call: tensor roofline of the gate/up kernel
         peak, src = measure_mxfp8_peak(device) if mx else (peaks["bf16_tflops"], peaks["source"] + " (burst cuBLAS bf16)")
         ach = 2.0 * T * k * K * N / (up_ms * 1e-3) / 1e12

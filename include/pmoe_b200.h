@@ -363,6 +363,8 @@ size_t pmoe_debug_bf16_workspace_extent(int M, int K, int N, int num_experts, in
  * the values below (0: one row block per tile, row-M kernels). Host only, no device work. */
 enum { PMOE_ROUTE_TOKEN_N_UP = 1, PMOE_ROUTE_TOKEN_N_DOWN = 2, PMOE_ROUTE_TWO_BLOCK_UP = 4, PMOE_ROUTE_CTA_PAIRS = 8 };
 int pmoe_debug_bf16_route(int M, int K, int N, int num_experts, int top_k, int bpc, int with_live_rows);
+/* ... and the mxfp8 split launcher, for x_scales that are 4-byte aligned. */
+int pmoe_debug_mxfp8_route(int M, int K, int N, int num_experts, int top_k, int bpc, int with_live_rows);
 /* ... and the backward pass: 1 = weight gradients on CTA pairs, 2 = the row-space GEMMs as well, or their sum; 4 = the
  * row-space GEMMs on the token-N kernels. */
 int pmoe_debug_backward_route(int T, int K, int N, int num_experts, int top_k);

@@ -62,6 +62,7 @@ SIGNATURES = {
     "pmoe_debug_wait_probe": (_i, [_vp]),
     "pmoe_debug_bf16_workspace_extent": (_sz, [_i] * 8),
     "pmoe_debug_bf16_route": (_i, [_i] * 7),
+    "pmoe_debug_mxfp8_route": (_i, [_i] * 7),
     "pmoe_debug_backward_route": (_i, [_i] * 5),
     "pmoe_debug_tokn_bulk_down": (_i, [_i] * 4),
 }

@@ -1205,10 +1205,28 @@ Workspace plan_workspace(int M, int K, int N, int sorted_num, int split) {
     return w;
 }
 
-// The split pipeline runs on the token-N kernels (figures in moe_tokn.cu), but with live_rows (M is then a capacity, which says
-// nothing about the piece size to choose) and where a row's scales cannot be read as words.
+// The split pipeline runs on the token-N kernels (moe_tokn.cu), but with live_rows (M is then a capacity, which says nothing
+// about the piece size to choose) and where a row's scales cannot be read as words. Their operand feed per MAC is smaller and
+// there is a second accumulator: from 192 MB of weights on they are the faster ones (whole call, token-N / row-M, 0.82 - 0.98
+// on 49 layers of 1 to 131 rows per expert; T = 5003, K = 2048, N = 1536, E = 128, top_k = 8 297 / 338 us; K = 3584, N = 768,
+// 700 rows per expert 323 / 365).
+// Below that the rounds decide: a call is a few rounds of tiles, a round of the CTA pairs takes some 0.6 of the time of a round
+// of single CTAs over the same contraction, but there are half as many pairs, and the launch that plans the work items costs
+// what 1000 elements of K cost. The weights of the sum are fitted to 181 such layers, timed with the weights in L2 and not: 57 of
+// them go to the row-M kernels, which makes the mean over both 0.955 of the row-M time, as all on the token-N kernels, without
+// their worst ones (K = 2560, N = 1792, 3 experts, 795 rows each 28 / 38 us; K = 1792, N = 512, 37 experts, 13 rows each 19 / 25).
+// The row-M CTA pairs of bpc = 2 are never the better ones by more than 8 % (60 layers, mean 0.84).
 bool take_token_n(const Problem &p) {
-    return token_n_enabled() && !call_extras().live_rows && (reinterpret_cast<uintptr_t>(p.x_scales) & 3) == 0;
+    if (!token_n_enabled() || call_extras().live_rows || (reinterpret_cast<uintptr_t>(p.x_scales) & 3) != 0) return false;
+    const long long rows = static_cast<long long>(p.M) * p.top_k, experts = std::min<long long>(p.E, rows);
+    if (token_n_forced() || p.bpc == 2 || 3 * experts * p.N * p.K / 2 > 192000000) return true;
+    const long long per = (rows + p.E - 1) / p.E, cap = tokn_cap(rows, p.E, true);
+    auto rounds = [&](long long row_tiles, int cols, int slots) { return (experts * row_tiles * (cols / 256) + slots - 1) / slots; };
+    const long long blocks = (per + BM - 1) / BM, pieces = (per + cap - 1) / cap;
+    const int sms = sm_count(), pairs = sms / 2, H = p.N / 2;
+    const long long single = 20 * rounds(blocks, p.N, sms) * p.K + 15 * rounds(blocks, p.K, sms) * H;
+    const long long paired = 12 * rounds(pieces, p.N, pairs) * p.K + 8 * rounds(pieces, p.K, pairs) * H + 20000;
+    return paired <= single;
 }
 
 int run(const Problem &p, void *workspace, cudaStream_t stream) {
@@ -1526,4 +1544,15 @@ extern "C" int pmoe_fused_moe_mxfp8_ex(const void *x, const void *x_scales, cons
                                            stream);
     extras = pmoe::CallExtras{};
     return rc;
+}
+
+extern "C" int pmoe_debug_mxfp8_route(int M, int K, int N, int num_experts, int top_k, int bpc, int with_live_rows) {
+    using namespace pmoe;
+    static const int32_t some = 0;
+    Problem p{};
+    p.M = M, p.K = K, p.N = N, p.E = num_experts, p.top_k = top_k, p.bpc = bpc, p.split = 1;
+    call_extras().live_rows = with_live_rows ? &some : nullptr;   // not read
+    const bool token_n = take_token_n(p);
+    call_extras() = CallExtras{};
+    return token_n ? PMOE_ROUTE_TOKEN_N_UP | PMOE_ROUTE_TOKEN_N_DOWN : bpc == 2 ? PMOE_ROUTE_CTA_PAIRS : 0;
 }

@@ -30,10 +30,8 @@
 // mxfp8 (block-scaled MMAs, N <= 192: two accumulators of 192 columns leave 128 for the scales): the scale tiles of the rows
 // come by TMA with their slot, those of w2 too; those of w have to be interleaved like the A tile and are put together by a
 // warp of their own. The chunk staged by the gate/up epilogue is the fp32 SwiGLU value (an MX block runs over two warps'
-// lanes); the store warps take a row a lane and quantise it as moe_mxfp8.cu does. Whole op against the one-CTA row-M kernels
-// (their operand feed per MAC is 1.25 times as large, and there is one accumulator), weights not in L2: 0.97 on 58 random
-// layers (0.84 - 1.14, the slower ones below 60 us); us: T = 5003, K = 2048, N = 1536, E = 128, top_k = 8 338 / 297;
-// 16 tokens 86 / 82; K = 3584, N = 768, 700 rows per expert 365 / 323.
+// lanes); the store warps take a row a lane and quantise it as moe_mxfp8.cu does. Which calls take these kernels and which the
+// row-M ones of moe_mxfp8.cu: take_token_n() there.
 #include <algorithm>
 #include <atomic>
 
@@ -1148,12 +1146,11 @@ int launch(const CUtensorMap &mw, const CUtensorMap &mrows, const CUtensorMap &m
 // of 20 KB at cap 64), compute wants wide accumulators (256 leaves TMEM for a second one); a cap below an expert's rows
 // reads its weights once per piece. Measured, us at cap 64 / 128 / 256: 28 rows 270 / 272 / 282; 41 rows 236 / 218 /
 // 221; 65 rows 423 / 359 / 377; 122 rows 188 / 148 / 149; 140 rows 1118 / 862 / 777.
-static int tokn_cap(const ToknProblem &p) {
-    const long long rows = static_cast<long long>(p.M) * p.top_k;
+int tokn_cap(long long rows, int E, bool mx) {
     // mxfp8: 192 leaves a second accumulator; 128 is never the better one (us at 128 / 192: K = 6400, N = 1280, 87 rows 459 /
     // 416; K = 3584, N = 10240, 106 rows 301 / 270; below 32 rows 64 and 192 differ by 3 % either way)
-    if (p.w_scales) return rows <= 32ll * p.E ? 64 : 192;
-    return rows <= 32ll * p.E ? 64 : rows <= 112ll * p.E ? 128 : 256;
+    if (mx) return rows <= 32ll * E ? 64 : 192;
+    return rows <= 32ll * E ? 64 : rows <= 112ll * E ? 128 : 256;
 }
 
 // How the down kernel adds its rows. Bulk reductions move 256 bytes an operation instead of 16, which counts at the power
@@ -1175,7 +1172,7 @@ size_t tokn_items_bytes(int sorted_num) {
 int run_tokn(const ToknProblem &p, void *act, void *items, int phases, cudaStream_t stream) {
     const int H = p.N / 2;
     const int max_blocks = p.sorted_num / BM;
-    const int cap = tokn_cap(p);
+    const int cap = tokn_cap(static_cast<long long>(p.M) * p.top_k, p.E, p.w_scales != nullptr);
     int32_t *count = static_cast<int32_t *>(items);
     int4 *items_end = static_cast<int4 *>(items) + 1 + 2 * static_cast<size_t>(max_blocks);
     int2 *row_info = reinterpret_cast<int2 *>(items_end);

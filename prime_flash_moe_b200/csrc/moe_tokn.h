@@ -24,6 +24,9 @@ struct ToknProblem {
 // bytes of the work-item list and the per-row tokens and weights for a routing table of `sorted_num` rows (16-byte aligned region)
 size_t tokn_items_bytes(int sorted_num);
 
+// rows of one work item at most, for `rows` routed rows over E experts
+int tokn_cap(long long rows, int E, bool mx);
+
 // act [sorted_num, N/2] (bf16 or e4m3) and items are regions of the call's workspace; `phases` as in phase_mask()
 int run_tokn(const ToknProblem &p, void *act, void *items, int phases, cudaStream_t stream);
 
