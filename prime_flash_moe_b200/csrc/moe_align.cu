@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) moe_align_hist_kernel(
 }
 
 __global__ void __launch_bounds__(kThreads) moe_align_scatter_kernel(
-    const int32_t *__restrict__ ids, int n, int E, int seg, const int *__restrict__ counts, int block_m,
+    const int32_t *ids, int n, int E, int seg, const int *counts, int block_m,
     int pad_to, int32_t *__restrict__ sorted, int32_t *__restrict__ expert_ids, int32_t *__restrict__ npp,
     int max_padded, int max_blocks) {
     extern __shared__ int sm[];
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kThreads) moe_align_scatter_kernel(
         int t = 0, p = 0;
 #pragma unroll 8
         for (int c = part; c < ctas; c += parts) {
-            const int v = __ldg(counts + static_cast<size_t>(c) * E + e);
+            const int v = counts[static_cast<size_t>(c) * E + e];
             t += v;
             p += c < me ? v : 0;
         }

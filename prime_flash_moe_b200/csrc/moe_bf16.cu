@@ -313,7 +313,7 @@ __device__ __forceinline__ void bulk_reduce_row(uint32_t acc, uint32_t lane_base
 
 // out[i] += bf16(acc32[i]): last launch of the single-GEMM-launch pipeline (split == 0)
 __global__ void __launch_bounds__(256)
-finalize_acc32_kernel(const float *__restrict__ acc32, __nv_bfloat16 *__restrict__ out, long long n8, int use_pdl) {
+finalize_acc32_kernel(const float *acc32, __nv_bfloat16 *__restrict__ out, long long n8, int use_pdl) {
     if (use_pdl) pdl_wait_primary();
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n8;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {

@@ -176,7 +176,7 @@ row_maps_kernel(const int32_t *__restrict__ sorted_ids, const int32_t *__restric
 
 // dx[t] = sum over the token's top_k routes of d_xs[row of the route] (fp32 sum, one rounding)
 __global__ void __launch_bounds__(256)
-combine_dx_kernel(const __nv_bfloat16 *__restrict__ dxs, const int32_t *__restrict__ inv, int top_k, int tokens,
+combine_dx_kernel(const __nv_bfloat16 *dxs, const int32_t *inv, int top_k, int tokens,
                   int K, __nv_bfloat16 *__restrict__ dx) {
     pdl_wait_primary();
     const int vec_per_row = K / 8;
@@ -818,7 +818,7 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // list, so that blocks without routed rows (routing tables padded to 256 rows) cost no tile slot in the static
 // schedule.
 __global__ void __launch_bounds__(1024)
-live_items_kernel(const int32_t *__restrict__ eblk, int E, int32_t *__restrict__ live_list,
+live_items_kernel(const int32_t *eblk, int E, int32_t *__restrict__ live_list,
                   int32_t *__restrict__ live_count) {
     __shared__ int sn[1024];
     pdl_wait_primary();
@@ -842,7 +842,7 @@ live_items_kernel(const int32_t *__restrict__ eblk, int E, int32_t *__restrict__
 // Work lists of the row-space GEMMs on CTA pairs, one CTA: for every expert its row blocks two by two (pair_list =
 // first block of each pair) and the odd last one (single_list); counts[0] = pairs, counts[1] = singles.
 __global__ void __launch_bounds__(1024)
-pair_items_kernel(const int32_t *__restrict__ eblk, int E, int32_t *__restrict__ pair_list,
+pair_items_kernel(const int32_t *eblk, int E, int32_t *__restrict__ pair_list,
                   int32_t *__restrict__ single_list, int32_t *__restrict__ counts) {
     __shared__ int sp[1024], ss[1024];
     pdl_wait_primary();

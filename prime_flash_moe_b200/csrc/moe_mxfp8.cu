@@ -167,7 +167,7 @@ __device__ __forceinline__ void issue_slot(uint32_t d, uint32_t a_smem, uint32_t
 // activation scales re-tiled into 512-byte tiles [block][K/128]. One warp per row.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-gather_rows_mxfp8_kernel(const uint8_t *__restrict__ x, const uint8_t *__restrict__ x_scales,
+gather_rows_mxfp8_kernel(const uint8_t *x, const uint8_t *x_scales,     // the quantiser may still be writing both
                          uint8_t *__restrict__ x_sorted, uint8_t *__restrict__ xsf_tiles, const Args a) {
     pdl_wait_primary();        // launched as a programmatic dependent of whatever the stream holds: the quantiser
     pdl_launch_dependents();   // the gate/up (or fused) kernel may set itself up; it waits for this grid before loading
@@ -184,8 +184,15 @@ gather_rows_mxfp8_kernel(const uint8_t *__restrict__ x, const uint8_t *__restric
         if (tok < 0 || tok >= a.M) continue;
         const int4 *src = reinterpret_cast<const int4 *>(x + static_cast<size_t>(tok) * a.K);
         int4 *dst = reinterpret_cast<int4 *>(x_sorted + static_cast<size_t>(row) * a.K);
-#pragma unroll 4
-        for (int ch = lane; ch < chunks; ch += 32) dst[ch] = __ldg(src + ch);
+        for (int ch = lane; ch < chunks; ch += 128) {      // four loads in flight
+            int4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (ch + 32 * u < chunks) v[u] = src[ch + 32 * u];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (ch + 32 * u < chunks) dst[ch + 32 * u] = v[u];
+        }
         const int r = row & 127;
         uint8_t *tiles = xsf_tiles + static_cast<size_t>(row >> 7) * (a.K / 128) * SF_TILE + (r & 31) * 16 + (r >> 5) * 4;
         const uint8_t *srow = x_scales + static_cast<size_t>(tok) * kblocks;
@@ -1120,7 +1127,7 @@ moe_fused_mxfp8_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
 
 // out[i] += bf16(acc32[i])
 __global__ void __launch_bounds__(256)
-finalize_acc32_mxfp8_kernel(const float *__restrict__ acc32, __nv_bfloat16 *__restrict__ out, long long n8,
+finalize_acc32_mxfp8_kernel(const float *acc32, __nv_bfloat16 *__restrict__ out, long long n8,
                             int use_pdl) {
     if (use_pdl) pdl_wait_primary();
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n8;

@@ -238,7 +238,7 @@ __device__ __forceinline__ void block_extents(const int32_t *sorted_ids, int c0,
     }
 }
 
-__device__ void plan_items(const int32_t *__restrict__ sorted_ids, const int32_t *__restrict__ expert_ids, int blocks,
+__device__ void plan_items(const int32_t *sorted_ids, const int32_t *expert_ids, int blocks,
                            int cap, int gran, int bpc, int4 *items_end, int32_t *item_count) {
     constexpr int kWarps = PLAN_THREADS / 32;
     __shared__ int s_first[kWarps];    // first run start of every warp's 32 blocks (or INT_MAX)
@@ -313,7 +313,7 @@ __device__ void plan_items(const int32_t *__restrict__ sorted_ids, const int32_t
 // mxfp8: the routed rows' scales (a word per row and 128 K elements) as 512-byte tiles [K / 128][max_blocks]; word w of a tile
 // is row w / 4 + 32 (w % 4). A thread keeps its row, so that neighbouring threads write neighbouring words and the eight
 // words of a sector of x_scales are read one after the other.
-__device__ __forceinline__ void tile_row_scales(const int32_t *__restrict__ sorted_ids, const uint32_t *__restrict__ x_scales,
+__device__ __forceinline__ void tile_row_scales(const int32_t *sorted_ids, const uint32_t *x_scales,
                                                 uint32_t *__restrict__ tiles, int blocks, int max_blocks, int M, int top_k,
                                                 int kt) {
     const int word = threadIdx.x & 127, part = threadIdx.x >> 7;      // four k ranges a CTA
@@ -324,18 +324,24 @@ __device__ __forceinline__ void tile_row_scales(const int32_t *__restrict__ sort
         if (tok < 0 || tok >= M) continue;      // padding rows only feed accumulator columns that nothing reads
         const uint32_t *src = x_scales + static_cast<size_t>(tok) * kt;
         const int end = min(kt, (part + 1) * per);
-#pragma unroll 4
-        for (int k = part * per; k < end; ++k) tiles[(static_cast<size_t>(k) * max_blocks + blk) * 128 + word] = __ldg(src + k);
+        for (int k = part * per; k < end; k += 4) {      // four loads in flight
+            uint32_t v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k + u < end) v[u] = src[k + u];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k + u < end) tiles[(static_cast<size_t>(k + u) * max_blocks + blk) * 128 + word] = v[u];
+        }
     }
 }
 
 // CTA 0 builds the work items; the other CTAs write every row's token and routing weight where the GEMM kernels find both
 // with one load instead of two dependent ones, and the scale tiles.
 __global__ void __launch_bounds__(PLAN_THREADS)
-plan_kernel(const int32_t *__restrict__ sorted_ids, const int32_t *__restrict__ expert_ids, const int32_t *__restrict__ npp,
-            const float *__restrict__ topk_weights, int M, int top_k, int sorted_num, int cap, int gran, int bpc,
-            int4 *items_end, int32_t *item_count, int2 *__restrict__ row_info, const uint32_t *__restrict__ x_scales,
-            uint32_t *__restrict__ sf_tiles, int kt) {
+plan_kernel(const int32_t *sorted_ids, const int32_t *expert_ids, const int32_t *npp, const float *topk_weights, int M,
+            int top_k, int sorted_num, int cap, int gran, int bpc, int4 *items_end, int32_t *item_count,
+            int2 *__restrict__ row_info, const uint32_t *x_scales, uint32_t *__restrict__ sf_tiles, int kt) {
     pdl_wait_primary();        // launched as a programmatic dependent of whatever the stream holds: the routing kernel
     pdl_launch_dependents();
     const int blocks = live_row_blocks(npp, sorted_num);
@@ -386,8 +392,8 @@ __device__ __forceinline__ void fetch_pairs(const Args &a, const Tile &w, int gr
         const int ch = grp + 2 * j;
         r[j] = make_int2(-1, 0);
         if (ch * CHUNK < w.rows) {
-            const int p = __ldg(a.sorted_ids + w.row0 + ch * CHUNK + lane);
-            if (p >= 0 && p < a.M) r[j] = make_int2(p, __float_as_int(__ldg(a.topk_weights + p)));
+            const int p = a.sorted_ids[w.row0 + ch * CHUNK + lane];
+            if (p >= 0 && p < a.M) r[j] = make_int2(p, __float_as_int(a.topk_weights[p]));
         }
     }
 }

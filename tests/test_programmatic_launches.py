@@ -1,0 +1,57 @@
+"""Kernels launched as programmatic dependents may be resident while the kernel before them still writes. What that one writes
+they must not read through the non-coherent path, whose data has to be constant while the kernel runs: no `const T
+*__restrict__` parameter (the compiler may then choose that path by itself) and no `__ldg` in a kernel that waits for its
+primary, nor in the device functions it may call."""
+import re
+from pathlib import Path
+
+import prime_flash_moe_b200
+
+CSRC = Path(prime_flash_moe_b200.__file__).parent / "csrc"
+
+# Launched once init_kernel has passed its own wait, so whatever ran before the backward pass is complete, and that is all they
+# take as constant.
+COMPLETE_BEFORE = {"row_maps_kernel", "gather_token_rows_kernel"}
+# files whose kernels are launched plainly
+PLAIN = {"moe_ep.cu"}
+
+
+def functions(text):
+    """(name, parameters, body) of every __global__ or __device__ function defined in `text`."""
+    text = re.sub(r"//[^\n]*|__launch_bounds__\([^()]*\)", "", text)
+    for m in re.finditer(r"__(?:global|device)__[^;{}()]*?(\w+)\(", text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[i], 0)
+            i += 1
+        params, rest = text[m.end():i - 1], text[i:].lstrip()
+        if not rest.startswith("{"):
+            continue
+        start = j = text.index("{", i)
+        depth = 0
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[j], 0)
+            j += 1
+            if depth == 0:
+                break
+        yield m.group(1), "__global__" in m.group(0), params, text[start:j]
+
+
+def test_programmatic_dependents_read_no_constant_path():
+    waiting, bad = set(), []
+    for path in sorted(CSRC.glob("*.cu*")):
+        for name, is_kernel, params, body in functions(path.read_text()):
+            waits = "pdl_wait_primary()" in body or "griddepcontrol.wait" in body
+            if is_kernel and waits:
+                waiting.add(name)
+            if path.name in PLAIN or name in COMPLETE_BEFORE or (is_kernel and not waits):
+                continue
+            if re.search(r"\bconst\b[^,]*\*\s*(const\s*)?__restrict__", params):
+                bad.append(f"{path.name}: {name} takes a const __restrict__ pointer")
+            if "__ldg(" in body:
+                bad.append(f"{path.name}: {name} loads by __ldg")
+    # the parser sees them: one of every file that launches programmatic dependents, and the exceptions
+    assert {"plan_kernel", "moe_tokn_kernel", "live_items_kernel", "pair_items_kernel", "combine_dx_kernel", "route_topk_kernel",
+            "quantize_mx_kernel", "moe_align_small_kernel", "moe_align_scatter_kernel", "gather_rows_mxfp8_kernel",
+            "finalize_acc32_kernel"} | COMPLETE_BEFORE <= waiting
+    assert not bad, "\n".join(bad)
