@@ -792,7 +792,7 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             auto release = [&]() {
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(mapa_shared(sm.misc(2 + buf), 0));
+                if (lane == 0) mbar_arrive_peer_tcgen05(mapa_shared(sm.misc(2 + buf), 0));
             };
             if (tma_stores(MODE)) {
                 const int m0 = m - lane;

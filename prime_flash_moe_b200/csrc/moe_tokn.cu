@@ -880,7 +880,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_shared(sm.tmem_empty(buf), 0));
+            if (lane == 0) mbar_arrive_peer_tcgen05(mapa_shared(sm.tmem_empty(buf), 0));
         }
         if (kMode == D_ACT) cp_async_wait_all();
     } else if (kUp && warp >= GATHER_WARP<kMx> && warp < GATHER_WARP<kMx> + GATHER_THREADS / 32) {
@@ -945,7 +945,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     ok = mbar_wait(sm.gathered(s), ph, status, ST_TIMEOUT_FULL);
                     if (!ok) break;
                     fence_proxy_async_smem();
-                    mbar_arrive_cluster(mapa_shared(sm.full(s), 0));
+                    mbar_arrive_peer_tcgen05(mapa_shared(sm.full(s), 0));
                     if (++s == a.stages) {
                         s = 0;
                         ph ^= 1;
@@ -999,7 +999,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     ok = mbar_wait(sm.scaled(b), ph, status, ST_TIMEOUT_FULL);
                     if (!ok) break;
                     fence_proxy_async_smem();
-                    mbar_arrive_cluster(mapa_shared(sm.sfa_full(b), 0));
+                    mbar_arrive_peer_tcgen05(mapa_shared(sm.sfa_full(b), 0));
                     if (++b == SFA_BATCHES) {
                         b = 0;
                         ph ^= 1;

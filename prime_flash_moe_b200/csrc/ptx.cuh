@@ -351,11 +351,21 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// Arrival on a barrier that may live in the peer CTA, with the default semantics (release, CTA scope). What it hands over is
-// an accumulator that has been read (tcgen05.wait::ld) or shared memory of this CTA whose writes have landed and been
-// fenced to the async proxy before: nothing that a release at cluster scope would still have to push out. That release
-// waits for every global access that the SM has in flight: one a k-step made a k-step 1.2 us instead of 0.35.
+// Arrival on a barrier that may live in the peer CTA, where a thread waits with cluster scope (mbar_wait_cluster)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same with the default semantics (release, CTA scope). A release at cluster scope waits for every global access that the
+// SM has in flight: one a k-step made a k-step 1.2 us instead of 0.35, one a tile, beside an epilogue's stores or reductions,
+// made calls 2 - 6 % longer (backward pass, K = 2048, N = 1536, 128 experts, 256 rows each 1024 / 1083 us; mxfp8, the same
+// layer, 5003 tokens 290 / 305). By the letter the order of the two CTAs then does not follow from the barrier's scopes. It
+// rests on what is handed over, all of which only the other CTA's tcgen05 instructions touch, issued after a wait on this barrier
+// and tcgen05.fence::after_thread_sync:
+//   - accumulator columns read by this warp: tcgen05.ld, tcgen05.wait::ld, tcgen05.fence::before_thread_sync, then the arrival
+//   - shared memory of this CTA whose writes have landed (cp.async, seen through a barrier of this CTA) and been fenced to the
+//     async proxy (fence.proxy.async) by the arriving thread
+// Nothing else may be handed over this way: a generic load or store of the other CTA would not be ordered.
+__device__ __forceinline__ void mbar_arrive_peer_tcgen05(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
@@ -372,8 +382,9 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
     return ok != 0;
 }
 // Bounded wait on a barrier on which threads of the peer CTA arrive (accumulator hand-back: once per tile). The ring
-// barriers of the pair kernels complete through TMA bytes and tcgen05.commit, not through another thread's writes:
-// they take the plain mbar_wait (a cluster-scope acquire per k-step made the same GEMM 10 % slower).
+// barriers of the pair kernels complete through TMA bytes, tcgen05.commit and mbar_arrive_peer_tcgen05, not through another
+// thread's writes to be read by this one: they take the plain mbar_wait (a cluster-scope acquire per k-step made the same GEMM
+// 10 % slower).
 static __device__ __noinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int *status, int code) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();

@@ -1,7 +1,4 @@
-"""Kernels launched as programmatic dependents may be resident while the kernel before them still writes. What that one writes
-they must not read through the non-coherent path, whose data has to be constant while the kernel runs: no `const T
-*__restrict__` parameter (the compiler may then choose that path by itself) and no `__ldg` in a kernel that waits for its
-primary, nor in the device functions it may call."""
+"""Rules of the CUDA sources that no run can show."""
 import re
 from pathlib import Path
 
@@ -38,6 +35,10 @@ def functions(text):
 
 
 def test_programmatic_dependents_read_no_constant_path():
+    """Kernels launched as programmatic dependents may be resident while the kernel before them still writes. What that one
+    writes they must not read through the non-coherent path, whose data has to be constant while the kernel runs: no `const T
+    *__restrict__` parameter (the compiler may then choose that path by itself) and no `__ldg` in a kernel that waits for its
+    primary, nor in the device functions it may call."""
     waiting, bad = set(), []
     for path in sorted(CSRC.glob("*.cu*")):
         for name, is_kernel, params, body in functions(path.read_text()):
@@ -55,3 +56,19 @@ def test_programmatic_dependents_read_no_constant_path():
             "quantize_mx_kernel", "moe_align_small_kernel", "moe_align_scatter_kernel", "gather_rows_mxfp8_kernel",
             "finalize_acc32_kernel"} | COMPLETE_BEFORE <= waiting
     assert not bad, "\n".join(bad)
+
+
+def test_scopes_of_arrivals_in_the_peer_cta():
+    """An arrival in the peer CTA releases at cluster scope where the wait acquires at cluster scope. The CTA-scope one hands
+    over drained accumulators (after tcgen05.fence::before_thread_sync) and shared memory fenced to the async proxy only."""
+    cluster, plain = set(), 0
+    for path in sorted(CSRC.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        assert ("mbar_wait_cluster(" in text) == ("mbar_arrive_cluster(" in text), path.name
+        if "mbar_arrive_cluster(" in text:
+            cluster.add(path.name)
+        for m in re.finditer(r"mbar_arrive_peer_tcgen05\(", text):
+            before = text[max(0, m.start() - 120):m.start()]
+            assert "tc_fence_before();" in before or "fence_proxy_async_smem();" in before, (path.name, before)
+            plain += 1
+    assert cluster == {"moe_bf16.cu", "moe_mxfp8.cu"} and plain >= 4
