@@ -71,6 +71,14 @@ def test_knobs(split, bn, wn, stages):
     assert O.max_rel_to_peak(out, ref) <= TOL
 
 
+@pytest.mark.parametrize("bn,wn", [(64, 4), (32, 8)])
+@pytest.mark.parametrize("stages", [1, 2, 3, 4])
+def test_knobs_of_the_row_m_kernels(bn, wn, stages, monkeypatch):
+    """The split pipeline's knobs select something in the row-M kernels only."""
+    monkeypatch.setenv("PMOE_TOKN", "0")
+    test_knobs(True, bn, wn, stages)
+
+
 def test_golden_vectors(golden):
     """Output of the reference's mxfp8 test oracle (test/test_mxfp8.py:50-77) stored in tests/golden. That
     oracle rounds the activation to bf16 before re-quantising it, the kernels (the reference's too)
@@ -190,6 +198,17 @@ def test_two_cta_pipeline(T, K, E, N, k, stages):
     assert O.max_rel_to_peak(pair, one.float()) <= TOL
 
 
+@pytest.mark.parametrize("stages", [1, 4])
+@pytest.mark.parametrize("T,K,E,N,k", [(8, 256, 1, 256, 1), (300, 512, 4, 512, 2), (128, 2048, 128, 1536, 8),
+                                       (2048, 2048, 32, 2048, 4), (1000, 7168, 8, 1024, 8)])
+def test_two_cta_pipeline_of_the_row_m_kernels(T, K, E, N, k, stages, monkeypatch):
+    """M = 256 pairs against the one-CTA kernels: what bpc = 2 runs with live_rows and with x_scales that are not words."""
+    from prime_flash_moe_b200 import capi
+    monkeypatch.setenv("PMOE_TOKN", "0")
+    assert capi.lib().pmoe_debug_mxfp8_route(T, K, N, E, k, 2, 0) == 8 and capi.lib().pmoe_debug_mxfp8_route(T, K, N, E, k, 1, 0) == 0
+    test_two_cta_pipeline(T, K, E, N, k, stages)
+
+
 def test_two_cta_rejects_fused_pipeline():
     import prime_flash_moe_b200 as P
     q, deq, ids, wts = quantised_case(64, 256, 2, 256, 2, seed=1)
@@ -219,7 +238,7 @@ def test_short_row_blocks(T, K, E, N, k, monkeypatch):
     assert O.max_rel_to_peak(short, full.float()) <= TOL
 
 
-def test_ex_entry_point_live_rows():
+def test_ex_entry_point_live_rows(bpc=1):
     """`pmoe_fused_moe_mxfp8_ex`: worst-case sized buffers with only the leading `live_rows` rows in use; rows beyond
     are neither read for a result nor zeroed."""
     import prime_flash_moe_b200 as P
@@ -237,15 +256,43 @@ def test_ex_entry_point_live_rows():
     wd = torch.zeros(cap, k, dtype=torch.float32, device=DEV)
     wd[:T] = wts.to(DEV)
     live = torch.tensor([T], dtype=torch.int32, device=DEV)
-    s, e, n = capi.moe_align(idd, E, 128, 1)
+    s, e, n = capi.moe_align(idd, E, 128, bpc)
     out = torch.full((cap, K), float("nan"), dtype=torch.bfloat16, device=DEV)
     capi.fused_moe_mxfp8(xd, sd, w1q.to(DEV), P.pack_scales_blocked(w1s).to(DEV), w2q.to(DEV),
-                         P.pack_scales_blocked(w2s).to(DEV), s, e, n, wd.view(-1), out, k, 128, 64, 4, 4, 1, True,
+                         P.pack_scales_blocked(w2s).to(DEV), s, e, n, wd.view(-1), out, k, 128, 64, 4, 4, bpc, True,
                          live_rows=live)
     torch.cuda.synchronize()
     assert O.max_rel_to_peak(out[:T].cpu(), ref) <= TOL
     assert torch.isnan(out[T:].float()).all()
     assert capi.device_status() == 0
+
+
+def test_ex_entry_point_live_rows_on_cta_pairs():
+    test_ex_entry_point_live_rows(bpc=2)
+
+
+@pytest.mark.parametrize("bpc", [1, 2])
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_scales_of_x_at_any_byte(offset, bpc, monkeypatch):
+    """x_scales need no alignment: words are read where they are 4-byte aligned, single bytes elsewhere (the row-M kernels,
+    also where PMOE_TOKN=1 asks for the others). The same result as from an aligned copy."""
+    from prime_flash_moe_b200 import capi
+    monkeypatch.setenv("PMOE_TOKN", "1")
+    T, K, E, N, k = 150, 512, 4, 512, 2
+    q, deq, ids, wts = quantised_case(T, K, E, N, k, seed=offset)
+    ref = O.moe_ref_fp32(deq["x"], deq["w1"], deq["w2"], ids, wts, requant_act=True)
+    whole, args = run_mine(q, ids, wts, True, bpc=bpc)
+    xs = args[1]
+    buf = torch.full((xs.numel() + 16,), 255, dtype=torch.uint8, device=DEV)      # 255: NaN, should a neighbour be read
+    view = buf[offset:offset + xs.numel()]
+    view.copy_(xs.view(torch.uint8).view(-1))
+    assert view.data_ptr() % 4 == offset % 4
+    out = torch.full((T, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    capi.fused_moe_mxfp8(args[0], view, *args[2:10], out, *args[11:])
+    torch.cuda.synchronize()
+    assert capi.device_status() == 0
+    assert O.max_rel_to_peak(out.cpu(), ref) <= TOL
+    assert O.max_rel_to_peak(out.cpu(), whole.float()) <= TOL
 
 
 @pytest.mark.parametrize("stages", [1, 2, 4])

@@ -56,7 +56,7 @@ def token_n(monkeypatch):
     monkeypatch.setenv("PMOE_TOKN", "1")
 
 
-# few rows per expert: pieces of at most 64 rows, more: 128, many: 192
+# few rows per expert: pieces of at most 64 rows, else of at most 192
 @pytest.mark.parametrize("bpc", [1, 2])
 @pytest.mark.parametrize("counts", [(1, 0, 2, 0), (31, 32, 33), (63, 65, 0, 1), (95, 97, 60), (127, 128, 129),
                                     (191, 192, 193), (0, 385, 300), (577, 1, 0)])
