@@ -694,6 +694,7 @@ moe_up_dual_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
         if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
+            long long issued = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
                 const Coord c = tile_coord(t, m_pairs, n_tiles);
@@ -714,6 +715,7 @@ moe_up_dual_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
                             tma_load_2d(sm.a(s, 0), &map_x, sm.full(s), ks * BK, p.blk[0] * BM);
                             if (p.nblk == 2) tma_load_2d(sm.a(s, 1), &map_x, sm.full(s), ks * BK, p.blk[1] * BM);
                         }
+                        ++issued;
                         if (++s == a.stages) {
                             s = 0;
                             ph ^= 1;
@@ -721,6 +723,7 @@ moe_up_dual_bf16_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
                     }
                 }
             }
+            if (!ok) drain_pair_fills(true, [&](int slot) { return sm.full(slot); }, a.stages, issued);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -1355,6 +1358,7 @@ moe_pair_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
+            long long issued = 0;
             bool ok = true;
             for (int t = first; t < num_tiles && ok; t += step) {
                 const Coord c = tile_coord(t, m_pairs, n_tiles);
@@ -1372,12 +1376,14 @@ moe_pair_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     if (leader) mbar_arrive_expect_tx(sm.full(s), 2 * PAIR_STAGE_BYTES);
                     tma_load_2d_pair(sm.a(s), &map_a, full_leader, ks * BK, blk * BM);
                     tma_load_2d_pair(sm.b(s), &map_b, full_leader, ks * BK, b_row);
+                    ++issued;
                     if (++s == a.stages) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
             }
+            if (!ok) drain_pair_fills(leader, [&](int slot) { return sm.full(slot); }, a.stages, issued);
         }
         __syncwarp();
     } else if (warp == 1) {

@@ -690,6 +690,7 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
+            long long issued = 0;
             bool ok = true;
             Tile next = fetch(first);
             for (int t = first; t < num_tiles && ok; t += step) {
@@ -720,12 +721,14 @@ moe_bwd_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         for (int j = 0; j < 2; ++j)
                             tma_load_2d_pair(sm.b(s) + j * BOX_BYTES, &map_b, full_leader, n0 + j * 64, krow);
                     }
+                    ++issued;
                     if (++s == PAIR_STAGES) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
             }
+            if (!ok) drain_pair_fills(leader, [&](int slot) { return sm.full(slot); }, PAIR_STAGES, issued);
         }
         __syncwarp();
     } else if (warp == 1) {

@@ -705,6 +705,7 @@ moe_pair_mxfp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
+            long long issued = 0;
             bool ok = true;
             for (int t = first; t < num_tiles && ok; t += step) {
                 const Coord c = tile_coord(t, m_pairs, n_tiles);
@@ -734,12 +735,14 @@ moe_pair_mxfp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                     tma_load_2d_pair(sm.sfa(s), &map_sfa, full_leader, 0, sfa0 + ks);
                     tma_load_2d_pair(sm.sfb(s), &map_sfb, full_leader, 0, sfb0 + ks);
                     tma_load_2d_pair(sm.sfb(s) + SF_TILE, &map_sfb, full_leader, 0, sfb1 + ks);
+                    ++issued;
                     if (++s == a.stages) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
             }
+            if (!ok) drain_pair_fills(leader, [&](int slot) { return sm.full(slot); }, a.stages, issued);
         }
         __syncwarp();
     } else if (warp == 1) {

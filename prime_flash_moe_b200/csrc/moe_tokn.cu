@@ -578,17 +578,7 @@ moe_tokn_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
                 if (!ok) issued = max(issued, before + early);
             }
-            if (!ok && leader) {
-                // give the copies already issued (both CTAs' bytes arrive here) a bounded time to land
-                const long long f0 = issued > a.stages ? issued - a.stages : 0;
-                for (long long f = f0; f < issued; ++f) {
-                    const uint32_t bar = sm.full(static_cast<int>(f % a.stages));
-                    const uint32_t parity = static_cast<uint32_t>((f / a.stages) & 1);
-                    const uint64_t t0 = globaltimer_ns();
-                    while (!mbar_try_wait(bar, parity))
-                        if (globaltimer_ns() - t0 > 20000000ull) break;
-                }
-            }
+            if (!ok) drain_pair_fills(leader, [&](int slot) { return sm.full(slot); }, a.stages, issued);
         }
         __syncwarp();
     } else if (warp == 1) {

@@ -400,6 +400,23 @@ static __device__ __noinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t par
     }
     return true;
 }
+// A producer whose wait ran out (or was given up because another role's did) gives its copies in flight a bounded time to land
+// before the CTA ends: the last `stages` of its `issued` fills, on the barriers full(slot). Both CTAs' bytes arrive on the even
+// CTA's barriers; the odd one's thread lets 1 ms pass, in case it has issued one more.
+template <typename Full>
+static __device__ void drain_pair_fills(bool leader, Full full, int stages, long long issued) {
+    if (!leader) {
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 1000000ull) {
+        }
+        return;
+    }
+    for (long long f = issued > stages ? issued - stages : 0; f < issued; ++f) {
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(full(static_cast<int>(f % stages)), static_cast<uint32_t>((f / stages) & 1)))
+            if (globaltimer_ns() - t0 > 20000000ull) break;      // 20 ms
+    }
+}
 // tile load whose completion bytes are signalled on `bar_cluster_addr`, which may live in the peer CTA
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar_cluster_addr,
                                                  int c0, int c1) {

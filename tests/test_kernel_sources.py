@@ -72,3 +72,15 @@ def test_scopes_of_arrivals_in_the_peer_cta():
             assert "tc_fence_before();" in before or "fence_proxy_async_smem();" in before, (path.name, before)
             plain += 1
     assert cluster == {"moe_bf16.cu", "moe_mxfp8.cu"} and plain >= 4
+
+
+def test_producers_wait_for_their_copies_in_flight():
+    """A kernel whose TMA producer gives up a wait lets the copies already issued land before it ends."""
+    seen = set()
+    for path in sorted(CSRC.glob("*.cu")):
+        for name, is_kernel, _, body in functions(path.read_text()):
+            if is_kernel and "ST_TIMEOUT_EMPTY" in body and "tma_load" in body:
+                seen.add(name)
+                assert re.search(r"drain_(pair_)?fills\(|20000000ull", body), f"{path.name}: {name}"
+    assert {"moe_tokn_kernel", "moe_up_dual_bf16_kernel", "moe_pair_bf16_kernel", "moe_pair_mxfp8_kernel", "moe_bwd_gemm_kernel",
+            "moe_bwd_pair_kernel", "moe_fused_bf16_kernel"} <= seen
