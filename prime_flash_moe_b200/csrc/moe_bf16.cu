@@ -1542,7 +1542,8 @@ int set_smem(Kernel k, size_t bytes) {
 
 // Byte offsets of the regions a call may carve out of its workspace. ONE function answers both "how large must
 // the workspace be" and "where does the launcher put each region", whatever PMOE_PREGATHER / PMOE_AGATHER / bpc
-// select at call time: every region is always reserved.
+// select at call time: every region is always reserved, although the token-N kernels use the activation and the work items
+// alone. The size is asked for without the number of experts, bpc or the extras of the call, which decide the kernels.
 //   split != 0: activation [sorted_num, H] bf16 | x_sorted [sorted_num, K] bf16 | pair list, tail list, counts |
 //               work items of the token-N kernels
 //   split == 0: fp32 accumulation buffer [M, K] (padded to 1024 bytes) | x_sorted [sorted_num, K] bf16
@@ -1605,7 +1606,7 @@ Decisions decide(const Problem &p) {
     const int up_tiles = p.N / 256;
     const bool one_wide_expert = call_extras().live_rows && p.E == 1 && p.bpc == 2 && p.K >= 3072 &&
                                  2 * up_tiles > sm_count() && up_tiles <= sm_count();
-    d.token_n = token_n_enabled() && !call_extras().out_rows && (token_n_forced() || !(long_rows || one_wide_expert));
+    d.token_n = token_n_enabled() && !call_extras().out_rows && (!(long_rows || one_wide_expert) || token_n_forced());
     if (d.token_n) return d;
     d.a_mode = a_operand_mode();
     // auto: the in-kernel LSU gather pays off when the row-gather pre-pass is a visible share of the step (its

@@ -61,7 +61,7 @@ __host__ __device__ constexpr bool is_wgrad(int mode) { return mode >= MODE_WGRA
 
 struct GArgs {
     int mode;
-    const int32_t *sorted_ids, *expert_ids, *npp;
+    const int32_t *sorted_ids;
     int sorted_num;
     const int32_t *eblk;          // MODE_WGRAD: first row block and one past the last routed row of every expert, [2 * E]
     const int32_t *items;         // row-space modes: the row blocks of this launch (pair kernel: first block of each
@@ -1174,7 +1174,7 @@ extern "C" int pmoe_fused_moe_bf16_backward_ex(const void *x, const void *w1, co
     if (int rc = bf16_map(&dw2_c, d_w2, static_cast<uint64_t>(E) * K, H, 32, "d_w2 (store)")) return rc;
 
     GArgs base{};
-    base.sorted_ids = sorted_token_ids, base.expert_ids = expert_ids, base.npp = num_tokens_post_padded;
+    base.sorted_ids = sorted_token_ids;
     base.sorted_num = sorted_num, base.eblk = eblk, base.topk_weights = topk_weights;
     base.top_k = top_k, base.tokens = T, base.E = E, base.H = H, base.N = N;
     // A row-space GEMM on CTA pairs is two launches: the pairs of row blocks, then the odd last blocks of the experts

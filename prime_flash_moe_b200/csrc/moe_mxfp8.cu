@@ -1229,7 +1229,7 @@ Workspace plan_workspace(int M, int K, int N, int sorted_num, int split) {
 bool take_token_n(const Problem &p) {
     if (!token_n_enabled() || call_extras().live_rows || (reinterpret_cast<uintptr_t>(p.x_scales) & 3) != 0) return false;
     const long long rows = static_cast<long long>(p.M) * p.top_k, experts = std::min<long long>(p.E, rows);
-    if (token_n_forced() || p.bpc == 2 || 3 * experts * p.N * p.K / 2 > 192000000) return true;
+    if (p.bpc == 2 || 3 * experts * p.N * p.K / 2 > 192000000 || token_n_forced()) return true;
     const long long per = (rows + p.E - 1) / p.E, cap = tokn_cap(rows, p.E, true);
     auto rounds = [&](long long row_tiles, int cols, int slots) { return (experts * row_tiles * (cols / 256) + slots - 1) / slots; };
     const long long blocks = (per + BM - 1) / BM, pieces = (per + cap - 1) / cap;
@@ -1275,7 +1275,8 @@ int run(const Problem &p, void *workspace, cudaStream_t stream) {
     a.xsf_tiles = xsf;
     a.acc32 = reinterpret_cast<float *>(base + w.acc32);
 
-    if (p.split && take_token_n(p)) {    // work items and row info (8.25 bytes a row and 16) in the place of x_sorted (K >= 256 a row)
+    // work items and row info (8.25 bytes a row and 16) in the place of x_sorted (K >= 256 bytes a row)
+    if (p.split && take_token_n(p)) {
         const ToknProblem t{p.x, p.w, p.w2, p.out, p.sorted_ids, p.expert_ids, p.npp, p.topk_weights, nullptr, nullptr,
                             p.top_k, p.M, p.K, p.N, p.E, p.sorted_num, p.bpc, p.x_scales, p.w_scales, p.w2_scales, xsf, act_sf};
         return run_tokn(t, act_q, x_sorted, phases, stream);

@@ -1203,8 +1203,7 @@ int run_tokn(const ToknProblem &p, void *act, void *items, int phases, cudaStrea
     const bool pdl = pdl_enabled();
     const long long max_items = std::min<long long>(2ll * max_blocks,
                                                     (static_cast<long long>(p.M) * p.top_k + cap - 1) / cap + max_blocks);
-    // The work items and the row info are built in every call, also in one whose phase mask leaves the row copy out:
-    // the kernels below index with them.
+    // The work items and the row info are built in every call, whatever the phase mask: the kernels below index with them.
     {
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1268,8 +1267,6 @@ int run_tokn(const ToknProblem &p, void *act, void *items, int phases, cudaStrea
     return PMOE_OK;
 }
 
-// Row-space GEMMs of the backward pass. Against the row-M kernels of moe_bwd_bf16.cu (128-row blocks, 48 KB of operands a
-// k-step on one CTA): see there.
 // Row-space GEMMs of the backward pass where an expert has few rows: every weight is read once and a row block costs what its
 // rows need, where the 128-row tile of the kernels in moe_bwd_bf16.cu multiplies padding (K = 2048, N = 1536, 128 experts, 64
 // rows each: recompute 154 -> 138 us, d_act 118 -> 103, d_xs 144 -> 140; where the line lies: there).

@@ -112,9 +112,8 @@ def test_an_expert_seen_in_separate_runs_and_holes_inside_a_block():
 @pytest.mark.parametrize("listed_twice", [False, True])
 @pytest.mark.parametrize("top_k,K", [(2, 2176), (3, 4096)])
 def test_rows_gathered_token_by_token(top_k, K, listed_twice):
-    """From 64 MB of activations on x is copied to the sorted rows token by token; some pairs are routed nowhere, some
-    tokens not at all; a hand-made table may list a pair in two rows. The row-M kernels, which gather by row, give the
-    expected result."""
+    """More than 64 MB of activations, gathered row by row inside the gate/up kernel; some pairs are routed nowhere, some
+    tokens not at all; a hand-made table may list a pair in two rows. The row-M kernels give the expected result."""
     import os
     from prime_flash_moe_b200 import capi
     N, E = 256, 40
@@ -139,7 +138,7 @@ def test_rows_gathered_token_by_token(top_k, K, listed_twice):
     outs = []
     for mode in ("1", "0"):
         os.environ["PMOE_TOKN"] = mode      # the fixture restores the variable
-        ws.fill_(255)                       # NaN where no row is copied
+        ws.fill_(255)                       # NaN where nothing is written
         outs.append(capi.fused_moe_bf16(x, w1, w2, s, e, n, wts, torch.empty_like(x), top_k, workspace=ws).float())
     torch.cuda.synchronize()
     assert capi.device_status() == 0
