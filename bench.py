@@ -1040,7 +1040,7 @@ def run_gpu_arm(args, impl):
         up_flops = 2.0 * rows_dominant * K * N
         achieved = up_flops / (per_kernel["up"] * 1e-3) / 1e12
         # DRAM bytes of one launch of that kernel, from the ncu captures summarised under profiles/
-        traffic = {("c1", "moe_pair_bf16_kernel<up>"): 2.713e9,
+        traffic = {("c1", "moe_tokn_kernel<up>"): 4.607e9, ("c1", "moe_pair_bf16_kernel<up>"): 2.713e9,
                    ("c2", "moe_up_bf16_kernel"): 1.112e9}.get(
             (args.config, path["up"])) if (not args.tokens and args.stages == 4 and args.warp_n == 4) else None
         roofline = {"kernel": path["up"], "down_kernel": path["down"], "includes": path["includes"], "bound": "tensor",

@@ -1580,19 +1580,19 @@ struct Decisions {
 Decisions decide(const Problem &p) {
     Decisions d{};
     // Token-N kernels, nearly whatever the size, since their gate/up kernel gathers the rows of x itself. Whole call against the
-    // row-M kernels: 0.70 - 1.00 on 110 random layers (K 1024 - 7168, N 512 - 26112, 1 - 253 experts, 1 - 33129 tokens; us:
-    // K = 2304, N = 768, 9 experts, 305 rows each 41 / 31; K = 4096, N = 3072, 32 experts, 4096 rows each 4388 / 4163), four at
-    // 1.02 - 1.07. Where the gate/up tiles are 1.0 to 2.0 times the CTA pairs (one round of the SMs, two of the pairs) they
-    // still win on 34 of 38 layers (0.77 - 0.99) and lose 1 - 8 % on the others (K = 3200, N = 3328, 6 rows on 6 experts 52 /
-    // 56), which no size tells apart.
+    // row-M kernels: 0.67 - 1.00 on 110 random layers (K 1024 - 7168, N 512 - 26112, 1 - 253 experts, 1 - 33129 tokens; us:
+    // K = 2304, N = 768, 9 experts, 305 rows each 40 / 30; K = 4096, N = 3072, 32 experts, 4096 rows each 4620 / 4346), one at
+    // 1.05. Where the gate/up tiles are 1.0 to 2.0 times the CTA pairs (one round of the SMs, two of the pairs) they still win
+    // on 34 of 38 layers (0.77 - 1.00) and lose 1 - 8 % on the others (K = 3200, N = 3328, 6 rows on 6 experts 52 / 56), which
+    // no size tells apart.
     // The largest calls stay with the two-block gate/up kernel, which gathers the rows as well, followed by the token-N down
     // kernel: these hold the power cap longest, and are the faster ones there (token-N / these, ms, runs of half a second back
-    // to back: K = 4096, N = 3072, 128 experts, 524288 rows, even 18.56 / 17.67, Zipf 17.87 / 17.65, on a hotter chip 19.52 /
-    // 18.43 and 19.17 / 18.71; with 32 experts 16.48 / 16.83). At 3.8e12 to 4.4e12 rows * K * N the two are level (0.96 - 1.03
-    // on six layers, one of them 1.02 on one chip and 0.98 on another), below that token-N is the faster one: 0.90 - 0.98 on
-    // 14 layers (K = 4096, N = 3072, 128 experts, 262144 rows 9.13 / 9.54; K = 6144, N = 5120, 64 experts, 65536 rows 6.08 /
-    // 6.82). On layers with 8 K <= 9 N and as CTA pairs (bpc = 2) it is level with or faster than the row-M kernels at every
-    // size (0.94 - 1.01 on eleven).
+    // to back: K = 4096, N = 3072, 128 experts, 524288 rows, even 18.56 / 17.67, Zipf 17.87 / 17.65; with 32 experts 16.48 /
+    // 16.83). At 3.8e12 to 4.4e12 rows * K * N the two are level (0.97 - 1.03 on six layers, one of them 1.02 on one chip and
+    // 0.98 on another), below that token-N is the faster one: 0.88 - 0.99 on 13 layers (K = 4096, N = 3072, 128 experts, 262144
+    // rows 9.13 / 9.54; K = 6144, N = 5120, 64 experts, 65536 rows 6.08 / 6.82). Layers with 8 K <= 9 N ran on token-N kernels
+    // with a row copy before, and bpc = 2 with long rows on the row-M pairs: 0.90 - 1.01 of either on eleven layers, the largest
+    // among them.
     // With live_rows M is a capacity, which says nothing about the rows in use. Token-N all the same (capacity 8192 or 16384,
     // 64 - 512 rows in use 0.41 - 0.97 of the row-M time), but for one wide expert as CTA pairs: its down kernel has K / 256
     // tiles whatever the rows, and its gate/up tiles take two rounds of the pairs where the single row block of a decode batch
